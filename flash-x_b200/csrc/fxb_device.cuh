@@ -120,6 +120,18 @@ __host__ __device__ inline bool extended_options(const DevParams &p)
            p.use_avisc || p.use_hybrid || p.nspec > 0;
 }
 
+// Option sets compiled into kernels: OPT_DEFAULT has the benchmark
+// configurations' choices (characteristic limiting, mc slopes where slopes are
+// used, HLLC, aux eint equation) as compile-time constants, OPT_ANY reads them
+// at run time.  The selections sit in every limiter and Riemann solve; without
+// them the 2-D FP64 PPM kernel spills 32 instead of 444 bytes per thread and
+// KH 2048^2 takes 0.94 instead of 1.09 ms per step (mixed 0.59 instead of 0.66).
+enum { OPT_ANY = 0, OPT_DEFAULT = 1 };
+__host__ __device__ inline bool default_options(const DevParams &p)
+{
+    return p.char_limiting && p.riemann == 4 && p.use_aux_eint && (p.order == 5 || p.limiter == LIM_MC);
+}
+
 // Fortran MIN/MAX with gfortran's argument order: mvar = a1; if (a2 < mvar) mvar = a2
 template <class R> __device__ __forceinline__ R fmin2(R a, R b) { return (b < a) ? b : a; }
 template <class R> __device__ __forceinline__ R fmax2(R a, R b) { return (b > a) ? b : a; }
@@ -218,7 +230,8 @@ template <class R> __device__ __forceinline__ Five<R> ldot(const Eig<R> &e, R xD
 // Inputs: the three states along the sweep (D, v1, v2, v3, P, EI order).
 // Output db[6] = limited slopes of D, v1, v2, v3, P (projected with R when
 // charLimiting) and EI (primitive).
-template <class R>
+// The limiter is selected once per cell, not once per wave.
+template <class R, int OPT = OPT_ANY>
 __device__ __forceinline__ void tvd_slope(const DevParams &prm, const Eig<R> &e,
                                           const R *VL, const R *V0, const R *VR, R db[6])
 {
@@ -226,20 +239,33 @@ __device__ __forceinline__ void tvd_slope(const DevParams &prm, const Eig<R> &e,
 #pragma unroll
     for (int k = 0; k < 6; k++) { dL[k] = V0[k] - VL[k]; dR[k] = VR[k] - V0[k]; }
     const R beta = R(prm.limited_beta);
-    if (prm.char_limiting) {
+    if (OPT == OPT_DEFAULT || prm.char_limiting) {
         Five<R> a = ldot(e, dL[0], dL[1], dL[2], dL[3], dL[4]);
         Five<R> b = ldot(e, dR[0], dR[1], dR[2], dR[3], dR[4]);
         R d[5];
+        // the five waves, and EI (primitive) into db[5]
+        auto all = [&](auto lim) {
 #pragma unroll
-        for (int w = 0; w < 5; w++) d[w] = limit(prm.limiter, w, -1, a.w[w], b.w[w], beta);
+            for (int w = 0; w < 5; w++) d[w] = lim(a.w[w], b.w[w]);
+            db[5] = lim(dL[5], dR[5]);
+        };
+        switch (OPT == OPT_DEFAULT ? (int)LIM_MC : prm.limiter) {
+        case LIM_MINMOD:  all([](R x, R y) { return lim_minmod(x, y); }); break;
+        case LIM_MC:      all([](R x, R y) { return lim_mc(x, y); }); break;
+        case LIM_VANLEER: all([](R x, R y) { return lim_vanleer(x, y); }); break;
+        case LIM_HYBRID:  // minmod on the acoustic/shear waves, mc on entropy and EI (hy_TVDslope.F90:146-174)
+            all([](R x, R y) { return lim_minmod(x, y); });
+            d[2] = lim_mc(a.w[2], b.w[2]);
+            db[5] = lim_mc(dL[5], dR[5]);
+            break;
+        default:          all([beta](R x, R y) { return lim_limited(x, y, beta); }); break;
+        }
         // R * delbar, summed over waves FASTLEFT..FASTRGHT (hy_DataReconstructNormalDir_PPM.F90:539-581)
         db[0] = (e.rho * d[0] + d[2]) + e.rho * d[4];
         db[1] = e.cf * d[4] - e.cf * d[0];
         db[2] = d[1];
         db[3] = d[3];
         db[4] = e.rp * d[0] + e.rp * d[4];
-        // gamc/game/eint keep primitive limiting; the hybrid choice is mc for them here (:165-170)
-        db[5] = (prm.limiter == LIM_HYBRID) ? lim_mc(dL[5], dR[5]) : limit(prm.limiter, -1, (int)EI, dL[5], dR[5], beta);
     } else {
         const int kind[6] = {D, VX, VY, VZ, P, EI};
 #pragma unroll
@@ -656,11 +682,11 @@ __device__ __noinline__ WenoPair<R> weno_scalar_body(int method, R I0, R I1, R I
 
 // WENO interface values of D, v1, v2, v3, P (characteristic when charLimiting)
 // and EI (primitive).  S[0..4][6] = Vmm, Vm, Vc, Vp, Vpp.
-template <class R>
+template <class R, int OPT = OPT_ANY>
 __device__ __forceinline__ void weno_interfaces(const DevParams &prm, const Eig<R> &e, const R S[5][6],
                                                 R vecL[6], R vecR[6])
 {
-    if (prm.char_limiting) {
+    if (OPT == OPT_DEFAULT || prm.char_limiting) {
         Five<R> w[5];
 #pragma unroll
         for (int s = 0; s < 5; s++) w[s] = ldot(e, S[s][0], S[s][1], S[s][2], S[s][3], S[s][4]);
@@ -981,7 +1007,7 @@ __device__ __forceinline__ int riemann_marquina(int dir, bool modified, const R 
 }
 
 // shock: the hybrid solver's face is next to a cell the shock detector marked
-template <class R, int EXT>
+template <class R, int EXT, int OPT = OPT_ANY>
 __device__ __forceinline__ int riemann(const DevParams &prm, int dir, const R *Vm, R gcL, R geL,
                                        const R *Vp, R gcR, R geR, R F[8], bool shock = false)
 {
@@ -992,7 +1018,8 @@ __device__ __forceinline__ int riemann(const DevParams &prm, int dir, const R *V
     const bool marq = EXT == 2 && (prm.riemann == 5 || prm.riemann == 7);
     // hy_getFaceFlux.F90:364-383: the hybrid solver is HLL next to a marked cell, HLLC elsewhere
     const bool hybr = EXT == 1 && prm.riemann == 8;
-    const bool hllc = !roe && !marq && (prm.riemann == 4 || (hybr && !shock)), llf = !roe && !marq && prm.riemann == 2;
+    const bool hllc = OPT == OPT_DEFAULT || (!roe && !marq && (prm.riemann == 4 || (hybr && !shock)));
+    const bool llf = OPT != OPT_DEFAULT && !roe && !marq && prm.riemann == 2;
     const R tiny = hllc ? R(prm.tiny) : R(1.e-32);
     if ((Vm[D] < tiny && Vm[D] > R(0)) || (Vp[D] < tiny && Vp[D] > R(0)) ||
         (Vm[P] < tiny && Vm[P] > R(0)) || (Vp[P] < tiny && Vp[P] > R(0))) {
@@ -1102,7 +1129,7 @@ __device__ __forceinline__ int riemann(const DevParams &prm, int dir, const R *V
         }
     }
     // aux internal-energy and volume fluxes (hy_getFaceFlux.F90:444-453)
-    if (prm.use_aux_eint) {
+    if (OPT == OPT_DEFAULT || prm.use_aux_eint) {
         if (F[0] > R(0)) { F[FVOL] = rdiv(F[0], Vm[D]); F[FEI] = F[0] * Vm[5]; }
         else             { F[FVOL] = rdiv(F[0], Vp[D]); F[FEI] = F[0] * Vp[5]; }
     } else { F[FVOL] = R(0); F[FEI] = R(0); }

@@ -126,7 +126,7 @@ __device__ __forceinline__ void set_err(int *err, int code) { atomicOr(err, code
 // the upwind transverse flux sigma of the direction other than dir at window
 // cell (wx, wy) (hy_upwindTransverseFlux), g its global-order 6-vector, eb its
 // eigensystem base; global order
-template <class R>
+template <class R, int OPT>
 __device__ __forceinline__ void sigma_other(const Args2D &a, const Smem2D<R> &s, int dir, int wx, int wy, const R g[6],
                                             const EigBase<R> &eb, R sg[6])
 {
@@ -136,14 +136,14 @@ __device__ __forceinline__ void sigma_other(const Args2D &a, const Smem2D<R> &s,
     rot(td, gm, m); rot(td, g, c); rot(td, gp, p);
     Eig<R> et;
     eigen_dir(eb, c[1], et);
-    trans_flux(et, m, c, p, a.prm.use_aux_eint != 0, sr);
+    trans_flux(et, m, c, p, OPT == OPT_DEFAULT || a.prm.use_aux_eint != 0, sr);
     unrot(td, sr, sg);
 }
 
 // Per-cell analysis along dir at a slope cell: the eigensystem and limited
 // slopes (PPM), and the upwind transverse flux sigma of the other direction
 // (hy_upwindTransverseFlux), which the state stage of dir subtracts.
-template <class R>
+template <class R, int OPT>
 __device__ __forceinline__ void analysis_stage(const Args2D &a, Smem2D<R> &s, int dir, int t, int wx, int wy,
                                                bool ppm)
 {
@@ -160,13 +160,13 @@ __device__ __forceinline__ void analysis_stage(const Args2D &a, Smem2D<R> &s, in
         rot(dir, gm, Vm); rot(dir, g, c); rot(dir, gp, Vp);
         Eig<R> e;
         eigen_dir(eb, c[1], e);
-        tvd_slope(a.prm, e, Vm, c, Vp, db);
+        tvd_slope<R, OPT>(a.prm, e, Vm, c, Vp, db);
 #pragma unroll
         for (int k = 0; k < 6; k++) s.DBF[k * NDB + t] = db[k];
     }
     if (KeepSig<R>::value) {
         R sg[6];
-        sigma_other(a, s, dir, wx, wy, g, eb, sg);
+        sigma_other<R, OPT>(a, s, dir, wx, wy, g, eb, sg);
 #pragma unroll
         for (int k = 0; k < 6; k++) s.SG[k][t] = sg[k];
     }
@@ -196,9 +196,9 @@ template <class R> __device__ __forceinline__ R divu2d(const Args2D &a, const Sm
 // face states of one cell along dir, with the transverse correction of the
 // other direction (hy_dataReconstOneStep.F90:931-936) and the negativity
 // fallback (:1131-1165); stores global-order Wp/Wm into s.W[.][t].
-template <class R, int EXT>
+template <class R, int EXT, int OPT>
 __device__ __forceinline__ void states_stage(const Args2D &a, Smem2D<R> &s, int dir, int t, int wx, int wy,
-                                             int dbi, int dbstep, R dtn, R hdtn, R hdtt, R hdt)
+                                             int dbi, int dbstep, R dtn, R hdtn, R hdtt, R hdt, int order)
 {
     const int ox = dir == 0, oy = dir == 1;
     R g[6], Vm[6], Vc[6], Vp[6], vecL[6], vecR[6], Wm[6], Wp[6];
@@ -219,12 +219,12 @@ __device__ __forceinline__ void states_stage(const Args2D &a, Smem2D<R> &s, int 
             // sigma of the other direction at this cell, times dt/2 dx_t, parked
             // in this thread's face-state slots until the transverse correction
             R sgo[6];
-            sigma_other(a, s, dir, wx, wy, g, eb, sgo);
+            sigma_other<R, OPT>(a, s, dir, wx, wy, g, eb, sgo);
 #pragma unroll
             for (int k = 0; k < 6; k++) s.W[k][t] = hdtt * sgo[k];
         }
     }
-    if (EXT && a.prm.order == 2) {
+    if (EXT && order == 2) {
         // MUSCL-Hancock: the cell's own slope, flattening and tracing in one step
         win6(s, wx - ox, wy - oy, g); rot(dir, g, Vm);
         win6(s, wx + ox, wy + oy, g); rot(dir, g, Vp);
@@ -238,11 +238,11 @@ __device__ __forceinline__ void states_stage(const Args2D &a, Smem2D<R> &s, int 
         mh_trace(a.prm, e, dtn, hdtn, Vm, Vc, Vp, F, wm, wp);
         unrot(dir, wm, Wm); unrot(dir, wp, Wp);
     } else {
-    if (a.prm.order == 5) {
+    if (order == 5) {
         R S[5][6];
 #pragma unroll
         for (int o = -2; o <= 2; o++) { win6(s, wx + o * ox, wy + o * oy, g); rot(dir, g, S[o + 2]); }
-        weno_interfaces(a.prm, e, S, vecL, vecR);
+        weno_interfaces<R, OPT>(a.prm, e, S, vecL, vecR);
 #pragma unroll
         for (int k = 0; k < 6; k++) { Vm[k] = S[1][k]; Vp[k] = S[3][k]; }
     } else {
@@ -317,7 +317,7 @@ template <class R> __device__ __forceinline__ R ener2d(const Args2D &a, int wx, 
     return (R)__ldg(a.in + DV_ENER * a.vstride + (long)my * a.nx + mx);
 }
 
-template <class R, int EXT>
+template <class R, int EXT, int OPT>
 __device__ __forceinline__ void faces_stage(const Args2D &a, Smem2D<R> &s, int dir, int t, int wl, int wr,
                                             int wxl, int wyl, int wxr, int wyr)
 {
@@ -330,7 +330,7 @@ __device__ __forceinline__ void faces_stage(const Args2D &a, Smem2D<R> &s, int d
         shock = shock_flag(a.shok, x0 + wxl, y0 + wyl, 0, a.nx, a.ny, 1, a.bc) +
                 shock_flag(a.shok, x0 + wxr, y0 + wyr, 0, a.nx, a.ny, 1, a.bc) > 0;
     }
-    int e = riemann<R, EXT>(a.prm, dir, VL, s.V[GC][wyl][wxl + XO], s.V[GE][wyl][wxl + XO],
+    int e = riemann<R, EXT, OPT>(a.prm, dir, VL, s.V[GC][wyl][wxl + XO], s.V[GE][wyl][wxl + XO],
                     VR, s.V[GC][wyr][wxr + XO], s.V[GE][wyr][wxr + XO], F, shock);
     if (e) set_err(a.err, e);
     if (EXT && a.prm.use_avisc) {
@@ -360,10 +360,13 @@ static_assert(sizeof(float) * 8 * WIN * WP % 128 == 0, "FP32 window size keeps t
 static_assert(sizeof(float) * (NF * NFC + 6 * NDB + 12 * NW + 4 * NDB) >= kWinBoxBytes,
               "FP32 staging area holds the FP64 window box");
 
-template <class R, int EXT>
+// ORDER: the reconstruction order, 0 where it is read at run time (extended
+// options); one order per kernel keeps PPM's and WENO's registers apart.
+template <class R, int EXT, int ORDER, int OPT>
 __global__ void __launch_bounds__(Threads2D<R>::value) __maxnreg__(Regs2D<R>::value)
 hydro2d_kernel(const __grid_constant__ Args2D a)
 {
+    const int order = ORDER ? ORDER : a.prm.order;
     extern __shared__ __align__(128) unsigned char smem_raw[];
     // 128-byte aligned base (the TMA destination); the launch adds 128 bytes
     unsigned char *base = smem_raw + ((128u - (smem_u32(smem_raw) & 127u)) & 127u);
@@ -473,24 +476,25 @@ hydro2d_kernel(const __grid_constant__ Args2D a)
     const R dtnx = R(dt_dx), hdtnx = R(0.5 * dt_dx);
     const R dtny = R(dt_dy), hdtny = R(0.5 * dt_dy);
     const R hdtx = R(uq[2]), hdty = R(uq[3]);
-    const bool ppm = a.prm.order == 3;     // PPM reads the slopes of its neighbours
+    const bool ppm = order == 3;           // PPM reads the slopes of its neighbours
 
     // ---- B: x slopes and sigma_y
     for (int t = tid; t < NDB; t += NT2) {
         int ii = t % (T2 + 4) - 2, jj = t / (T2 + 4);
-        analysis_stage(a, s, 0, t, ii + 3, jj + 3, ppm);
+        analysis_stage<R, OPT>(a, s, 0, t, ii + 3, jj + 3, ppm);
     }
     __syncthreads();
     // ---- C: x face states
     for (int t = tid; t < NW; t += NT2) {
         int ii = t % (T2 + 2) - 1, jj = t / (T2 + 2);
-        states_stage<R, EXT>(a, s, 0, t, ii + 3, jj + 3, jj * (T2 + 4) + ii + 2, 1, dtnx, hdtnx, hdty, R(0.5 * dt));
+        states_stage<R, EXT, OPT>(a, s, 0, t, ii + 3, jj + 3, jj * (T2 + 4) + ii + 2, 1, dtnx, hdtnx, hdty, R(0.5 * dt),
+                                  order);
     }
     __syncthreads();
     // ---- D: x faces
     for (int t = tid; t < NFC; t += NT2) {
         int fi = t % (T2 + 1), jj = t / (T2 + 1);
-        faces_stage<R, EXT>(a, s, 0, t, jj * (T2 + 2) + fi, jj * (T2 + 2) + fi + 1, fi + 2, jj + 3, fi + 3, jj + 3);
+        faces_stage<R, EXT, OPT>(a, s, 0, t, jj * (T2 + 2) + fi, jj * (T2 + 2) + fi + 1, fi + 2, jj + 3, fi + 3, jj + 3);
         if (EXT && a.fd[0] && (fi < T2 || tx0 + T2 == a.nx))   // the species' mass fluxes
             ((R *)a.fd[0])[(long)(ty0 + jj) * (a.nx + 1) + tx0 + fi] = s.DBF[FD * NFC + t];
     }
@@ -526,19 +530,20 @@ hydro2d_kernel(const __grid_constant__ Args2D a)
     // ---- F: y slopes and sigma_x
     for (int t = tid; t < NDB; t += NT2) {
         int ii = t % T2, jj = t / T2 - 2;
-        analysis_stage(a, s, 1, t, ii + 3, jj + 3, ppm);
+        analysis_stage<R, OPT>(a, s, 1, t, ii + 3, jj + 3, ppm);
     }
     __syncthreads();
     // ---- G: y face states
     for (int t = tid; t < NW; t += NT2) {
         int ii = t % T2, jj = t / T2 - 1;
-        states_stage<R, EXT>(a, s, 1, t, ii + 3, jj + 3, (jj + 2) * T2 + ii, T2, dtny, hdtny, hdtx, R(0.5 * dt));
+        states_stage<R, EXT, OPT>(a, s, 1, t, ii + 3, jj + 3, (jj + 2) * T2 + ii, T2, dtny, hdtny, hdtx, R(0.5 * dt),
+                                  order);
     }
     __syncthreads();
     // ---- H: y faces
     for (int t = tid; t < NFC; t += NT2) {
         int ii = t % T2, fj = t / T2;
-        faces_stage<R, EXT>(a, s, 1, t, fj * T2 + ii, (fj + 1) * T2 + ii, ii + 3, fj + 2, ii + 3, fj + 3);
+        faces_stage<R, EXT, OPT>(a, s, 1, t, fj * T2 + ii, (fj + 1) * T2 + ii, ii + 3, fj + 2, ii + 3, fj + 3);
         if (EXT && a.fd[1] && (fj < T2 || ty0 + T2 == a.ny))
             ((R *)a.fd[1])[(long)(ty0 + fj) * a.nx + tx0 + ii] = s.DBF[FD * NFC + t];
     }
@@ -627,6 +632,35 @@ hydro2d_kernel(const __grid_constant__ Args2D a)
         double m = red[0];
         for (int w = 1; w < NT2 / 32; w++) m = fmax(m, red[w]);
         atomicMax(a.rate_max, (unsigned long long)__double_as_longlong(m));
+    }
+}
+
+// set-up and launch of the instantiation for a step's options
+template <class R, class F> cudaError_t each_hydro2d(F f)
+{
+    cudaError_t e = f(hydro2d_kernel<R, 0, 3, OPT_DEFAULT>);
+    if (e == cudaSuccess) e = f(hydro2d_kernel<R, 0, 3, OPT_ANY>);
+    if (e == cudaSuccess) e = f(hydro2d_kernel<R, 0, 5, OPT_DEFAULT>);
+    if (e == cudaSuccess) e = f(hydro2d_kernel<R, 0, 5, OPT_ANY>);
+    if (e == cudaSuccess) e = f(hydro2d_kernel<R, 1, 0, OPT_ANY>);
+    if (e == cudaSuccess) e = f(hydro2d_kernel<R, 2, 0, OPT_ANY>);
+    return e;
+}
+template <class R> __global__ void flat2d_kernel(const Args2D a, R *flat);
+template <class R> void launch_hydro2d_t(const Args2D &a, dim3 grid, cudaStream_t s)
+{
+    const int nt = Threads2D<R>::value, sm = smem2d_bytes<R>();
+    if (a.prm.flattening) flat2d_kernel<R><<<148 * 8, 256, 0, s>>>(a, (R *)a.flat);
+    if (marquina_solver(a.prm))                          // Marquina solvers (with any other option)
+        hydro2d_kernel<R, 2, 0, OPT_ANY><<<grid, nt, sm, s>>>(a);
+    else if (extended_options(a.prm) || a.prm.use_gravity)   // Roe, contact steepening, MUSCL-Hancock, 2-D gravity
+        hydro2d_kernel<R, 1, 0, OPT_ANY><<<grid, nt, sm, s>>>(a);
+    else if (a.prm.order == 5) {
+        if (default_options(a.prm)) hydro2d_kernel<R, 0, 5, OPT_DEFAULT><<<grid, nt, sm, s>>>(a);
+        else hydro2d_kernel<R, 0, 5, OPT_ANY><<<grid, nt, sm, s>>>(a);
+    } else {
+        if (default_options(a.prm)) hydro2d_kernel<R, 0, 3, OPT_DEFAULT><<<grid, nt, sm, s>>>(a);
+        else hydro2d_kernel<R, 0, 3, OPT_ANY><<<grid, nt, sm, s>>>(a);
     }
 }
 
