@@ -58,7 +58,7 @@ template <> __device__ __forceinline__ float rdiv<float>(float a, float b) { ret
 // and RN(q + r y) = RN(a/b).  copysign gives a zero quotient the sign of
 // a / b.  Five FP64 operations per quotient after one division for y.
 // Valid for finite nonzero b and quotients and remainders in the normal
-// range (|a| >= 2^-960 or a = 0).  FP32: the fast division.
+// range (|a| >= 2^-960 or a = 0).  FP32: a times the reciprocal.
 template <class R> __device__ __forceinline__ R rdiv_y(R a, R b, R y);
 template <> __device__ __forceinline__ double rdiv_y<double>(double a, double b, double y)
 {
@@ -67,7 +67,19 @@ template <> __device__ __forceinline__ double rdiv_y<double>(double a, double b,
     q = fma(fma(-b, q, a), y, q);
     return copysign(q, a * y);
 }
-template <> __device__ __forceinline__ float rdiv_y<float>(float a, float b, float y) { return __fdividef(a, b); }
+template <> __device__ __forceinline__ float rdiv_y<float>(float a, float b, float y) { return a * y; }
+// y = 1 / b for rdiv_y.  FP32: the hardware reciprocal (PTX rcp.approx.ftz.f32,
+// error at most 1 ulp), so that a quotient is within the 2 ulp of the fast
+// division (PTX div.approx.f32) at one multiplication instead of a reciprocal,
+// a multiplication and the scaling of large denominators each.
+template <class R> __device__ __forceinline__ R rcp_y(R b);
+template <> __device__ __forceinline__ double rcp_y<double>(double b) { return 1.0 / b; }
+template <> __device__ __forceinline__ float rcp_y<float>(float b)
+{
+    float y;
+    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(b));
+    return y;
+}
 template <class R> __device__ __forceinline__ R rsqrt_(R a);
 template <> __device__ __forceinline__ double rsqrt_<double>(double a) { return sqrt(a); }
 // FP32 (mixed precision): the hardware approximation (PTX sqrt.approx.f32,
@@ -78,6 +90,48 @@ template <> __device__ __forceinline__ float rsqrt_<float>(float a)
     float r;
     asm("sqrt.approx.f32 %0, %1;" : "=f"(r) : "f"(a));
     return r;
+}
+
+// The reciprocals of a group of WENO denominators for rdiv_y.  FP64: without
+// a branch per value.  The division operator tests its operands and branches
+// to a slow path, so independent divisions run one after the other; here the
+// sequences of the group interleave and one test covers them all.  Two
+// Newton-Raphson steps on the hardware approximation (PTX rcp.approx.ftz.f64)
+// leave y within one ulp of 1/b; there the remainder 1 - b y is exact in one
+// FMA and a third step returns RN(1/b) unless b's significand is all ones
+// (P. Markstein, IBM J. Res. Dev. 34(1), 1990; tests/test_reciprocal.py).  A
+// group with a value outside 2^-400 .. 2^400, or with such a significand,
+// takes the division operator.  RT 128^3 FP64 1.63 -> 1.55 ms per step; the
+// eigensystem's and the Riemann solver's divisions, which are not the chain
+// their kernels wait for, got slower this way (KH 2048^2 0.93 -> 0.99 ms).
+__device__ __forceinline__ double rcp64(double b)
+{
+    double y;
+    asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(b));
+    y = fma(y, fma(-b, y, 1.0), y);
+    y = fma(y, fma(-b, y, 1.0), y);
+    return fma(y, fma(-b, y, 1.0), y);
+}
+__device__ __forceinline__ bool rcp64_ok(double b)
+{
+    const unsigned h = (unsigned)__double2hiint(b) & 0x7fffffffu;
+    return h - 0x26f00000u < 0x32000000u && ((h | 0xfff00000u) & (unsigned)__double2loint(b)) != 0xffffffffu;
+}
+static __device__ __noinline__ double rcp64_slow(double b) { return 1.0 / b; }
+template <int N> __device__ __forceinline__ void recips(const double (&b)[N], double (&y)[N])
+{
+    bool ok = true;
+#pragma unroll
+    for (int i = 0; i < N; i++) { y[i] = rcp64(b[i]); ok = ok && rcp64_ok(b[i]); }
+    if (!ok) {
+#pragma unroll
+        for (int i = 0; i < N; i++) y[i] = rcp64_slow(b[i]);
+    }
+}
+template <int N> __device__ __forceinline__ void recips(const float (&b)[N], float (&y)[N])
+{
+#pragma unroll
+    for (int i = 0; i < N; i++) y[i] = rcp_y(b[i]);
 }
 
 // Division by the literal constants 3, 6 and 12 of the PPM formulas.
@@ -186,13 +240,13 @@ template <class R> struct EigBase {
 };
 template <class R> __device__ __forceinline__ bool eigen_base(R rho, R p, R gamc, EigBase<R> &b)
 {
-    const R dinv = rdiv(R(1), rho);
+    const R dinv = rcp_y(rho);
     R a2 = rdiv_y(gamc * p, rho, dinv);
     if (a2 <= R(0)) return false;
     R cf = rsqrt_(a2);
     R aa2 = cf * cf;
-    b.a2inv = rdiv(R(1), aa2);
-    b.ahinv = rdiv(R(.5), cf);
+    b.a2inv = rcp_y(aa2);
+    b.ahinv = sizeof(R) == 8 ? rdiv(R(.5), cf) : R(.5) * rcp_y(cf);
     R Na = R(.5) * b.a2inv;
     b.lp = dinv * Na;
     b.cf = cf; b.rho = rho; b.rp = rho * aa2;
@@ -625,7 +679,6 @@ __device__ __forceinline__ void weno_scalar(int method, R I0, R I1, R I2, R I3, 
 template <class R>
 __device__ __noinline__ WenoPair<R> weno_scalar_body(int method, R I0, R I1, R I2, R I3, R I4)
 {
-    R vr, vl;
     const R c6 = R(6.);
     const R p00 = R(2.) / c6, p01 = R(-7.) / c6, p02 = R(11.) / c6;
     const R p10 = R(-1.) / c6, p11 = R(5.) / c6, p12 = R(2.) / c6;
@@ -650,64 +703,81 @@ __device__ __noinline__ WenoPair<R> weno_scalar_body(int method, R I0, R I1, R I
     const R tiny = R(1.e-36);
     // every quotient below shares its denominator with another: the
     // indicators' with the other side's, the sums' with the other weights
-    const R d0 = tiny + b0, d1 = tiny + b1, d2 = tiny + b2;
-    const R y0 = rdiv(R(1), d0), y1 = rdiv(R(1), d1), y2 = rdiv(R(1), d2);
-    R a0, a1, a2, s, ys;
-    // i+1/2, gammas (0.1, 0.6, 0.3)
+    const R d[3] = {tiny + b0, tiny + b1, tiny + b2};
+    R y[3];
+    recips(d, y);
+    // weights of i+1/2, gammas (0.1, 0.6, 0.3), and of i-1/2, gammas (0.3, 0.6, 0.1)
+    R a[3], c[3];
     if (method == 2) {
-        R tau = fabs(b0 - b2);
-        a0 = R(0.1) * (R(1.) + rdiv_y(tau, d0, y0));
-        a1 = R(0.6) * (R(1.) + rdiv_y(tau, d1, y1));
-        a2 = R(0.3) * (R(1.) + rdiv_y(tau, d2, y2));
+        const R tau = fabs(b0 - b2);
+        const R t0 = R(1.) + rdiv_y(tau, d[0], y[0]), t1 = R(1.) + rdiv_y(tau, d[1], y[1]),
+                t2 = R(1.) + rdiv_y(tau, d[2], y[2]);
+        a[0] = R(0.1) * t0; a[1] = R(0.6) * t1; a[2] = R(0.3) * t2;
+        c[0] = R(0.3) * t0; c[1] = R(0.6) * t1; c[2] = R(0.1) * t2;
     } else {
-        a0 = rdiv_y(R(0.1), d0, y0); a1 = rdiv_y(R(0.6), d1, y1); a2 = rdiv_y(R(0.3), d2, y2);
+        a[0] = rdiv_y(R(0.1), d[0], y[0]); a[1] = rdiv_y(R(0.6), d[1], y[1]); a[2] = rdiv_y(R(0.3), d[2], y[2]);
+        c[0] = rdiv_y(R(0.3), d[0], y[0]); c[1] = a[1]; c[2] = rdiv_y(R(0.1), d[2], y[2]);
     }
-    s = a0 + a1 + a2;
-    ys = rdiv(R(1), s);
-    vr = rdiv_y(a0, s, ys) * w5p0 + rdiv_y(a1, s, ys) * w5p1 + rdiv_y(a2, s, ys) * w5p2;
-    // i-1/2, gammas (0.3, 0.6, 0.1)
-    if (method == 2) {
-        R tau = fabs(b0 - b2);
-        a0 = R(0.3) * (R(1.) + rdiv_y(tau, d0, y0));
-        a1 = R(0.6) * (R(1.) + rdiv_y(tau, d1, y1));
-        a2 = R(0.1) * (R(1.) + rdiv_y(tau, d2, y2));
-    } else {
-        a0 = rdiv_y(R(0.3), d0, y0); a1 = rdiv_y(R(0.6), d1, y1); a2 = rdiv_y(R(0.1), d2, y2);
-    }
-    s = a0 + a1 + a2;
-    ys = rdiv(R(1), s);
-    vl = rdiv_y(a0, s, ys) * w5m0 + rdiv_y(a1, s, ys) * w5m1 + rdiv_y(a2, s, ys) * w5m2;
+    const R s[2] = {a[0] + a[1] + a[2], c[0] + c[1] + c[2]};
+    R ys[2];
+    recips(s, ys);
+    const R vr = rdiv_y(a[0], s[0], ys[0]) * w5p0 + rdiv_y(a[1], s[0], ys[0]) * w5p1 + rdiv_y(a[2], s[0], ys[0]) * w5p2;
+    const R vl = rdiv_y(c[0], s[1], ys[1]) * w5m0 + rdiv_y(c[1], s[1], ys[1]) * w5m1 + rdiv_y(c[2], s[1], ys[1]) * w5m2;
     return WenoPair<R>{vr, vl};
 }
 
 // WENO interface values of D, v1, v2, v3, P (characteristic when charLimiting)
-// and EI (primitive).  S[0..4][6] = Vmm, Vm, Vc, Vp, Vpp.
+// and EI (primitive).  ld(v, o) gives the sweep-order variable v of the cell
+// o = 0 .. 4 of the stencil (Vmm, Vm, Vc, Vp, Vpp); the waves are taken one at
+// a time, so that only the values of one or two variables are live at once
+// (2-D FP64 kernel, 816 x 624: 223 -> 214 us per step).
+template <class R, int OPT = OPT_ANY, class F>
+__device__ __forceinline__ void weno_interfaces_of(const DevParams &prm, const Eig<R> &e, F ld, R vecL[6], R vecR[6])
+{
+    const int m = prm.weno_method;
+    R I[5], cr[3], cl[3];
+#pragma unroll
+    for (int o = 0; o < 5; o++) I[o] = ld(5, o);
+    weno_scalar(m, I[0], I[1], I[2], I[3], I[4], vecR[5], vecL[5]);
+#pragma unroll
+    for (int v = 2; v <= 3; v++) {         // the shear waves are v2 and v3 themselves
+#pragma unroll
+        for (int o = 0; o < 5; o++) I[o] = ld(v, o);
+        weno_scalar(m, I[0], I[1], I[2], I[3], I[4], vecR[v], vecL[v]);
+    }
+    if (OPT == OPT_DEFAULT || prm.char_limiting) {
+        // left-eigenvector products as in ldot: u - c, entropy, u + c
+#pragma unroll
+        for (int o = 0; o < 5; o++) I[o] = e.lp * ld(4, o) - e.ahinv * ld(1, o);
+        weno_scalar(m, I[0], I[1], I[2], I[3], I[4], cr[0], cl[0]);
+#pragma unroll
+        for (int o = 0; o < 5; o++) I[o] = ld(0, o) - e.a2inv * ld(4, o);
+        weno_scalar(m, I[0], I[1], I[2], I[3], I[4], cr[1], cl[1]);
+#pragma unroll
+        for (int o = 0; o < 5; o++) I[o] = e.ahinv * ld(1, o) + e.lp * ld(4, o);
+        weno_scalar(m, I[0], I[1], I[2], I[3], I[4], cr[2], cl[2]);
+        vecR[0] = (e.rho * cr[0] + cr[1]) + e.rho * cr[2];
+        vecR[1] = e.cf * cr[2] - e.cf * cr[0];
+        vecR[4] = e.rp * cr[0] + e.rp * cr[2];
+        vecL[0] = (e.rho * cl[0] + cl[1]) + e.rho * cl[2];
+        vecL[1] = e.cf * cl[2] - e.cf * cl[0];
+        vecL[4] = e.rp * cl[0] + e.rp * cl[2];
+    } else {
+#pragma unroll
+        for (int n = 0; n < 3; n++) {
+            const int v = n == 2 ? 4 : n;
+#pragma unroll
+            for (int o = 0; o < 5; o++) I[o] = ld(v, o);
+            weno_scalar(m, I[0], I[1], I[2], I[3], I[4], vecR[v], vecL[v]);
+        }
+    }
+}
+// the same from S[0..4][6] = Vmm, Vm, Vc, Vp, Vpp
 template <class R, int OPT = OPT_ANY>
 __device__ __forceinline__ void weno_interfaces(const DevParams &prm, const Eig<R> &e, const R S[5][6],
                                                 R vecL[6], R vecR[6])
 {
-    if (OPT == OPT_DEFAULT || prm.char_limiting) {
-        Five<R> w[5];
-#pragma unroll
-        for (int s = 0; s < 5; s++) w[s] = ldot(e, S[s][0], S[s][1], S[s][2], S[s][3], S[s][4]);
-        R cr[5], cl[5];
-#pragma unroll
-        for (int n = 0; n < 5; n++)
-            weno_scalar(prm.weno_method, w[0].w[n], w[1].w[n], w[2].w[n], w[3].w[n], w[4].w[n], cr[n], cl[n]);
-        vecR[0] = (e.rho * cr[0] + cr[2]) + e.rho * cr[4];
-        vecR[1] = e.cf * cr[4] - e.cf * cr[0];
-        vecR[2] = cr[1]; vecR[3] = cr[3];
-        vecR[4] = e.rp * cr[0] + e.rp * cr[4];
-        vecL[0] = (e.rho * cl[0] + cl[2]) + e.rho * cl[4];
-        vecL[1] = e.cf * cl[4] - e.cf * cl[0];
-        vecL[2] = cl[1]; vecL[3] = cl[3];
-        vecL[4] = e.rp * cl[0] + e.rp * cl[4];
-    } else {
-#pragma unroll
-        for (int n = 0; n < 5; n++)
-            weno_scalar(prm.weno_method, S[0][n], S[1][n], S[2][n], S[3][n], S[4][n], vecR[n], vecL[n]);
-    }
-    weno_scalar(prm.weno_method, S[0][5], S[1][5], S[2][5], S[3][5], S[4][5], vecR[5], vecL[5]);
+    weno_interfaces_of<R, OPT>(prm, e, [&](int v, int o) { return S[o][v]; }, vecL, vecR);
 }
 
 // Reconstructed face values of the (constant) gravity component along the
@@ -1012,8 +1082,10 @@ __device__ __forceinline__ int riemann(const DevParams &prm, int dir, const R *V
                                        const R *Vp, R gcR, R geR, R F[8], bool shock = false)
 {
     const R velNL = Vm[1 + dir], velNR = Vp[1 + dir];
-    const R aL2 = rdiv(gcL * Vm[P], Vm[D]);
-    const R aR2 = rdiv(gcR * Vp[P], Vp[D]);
+    // FP32 shares the densities' reciprocals with the volume flux; FP64 divides
+    const R yDL = sizeof(R) == 4 ? rcp_y(Vm[D]) : R(0), yDR = sizeof(R) == 4 ? rcp_y(Vp[D]) : R(0);
+    const R aL2 = sizeof(R) == 4 ? gcL * Vm[P] * yDL : rdiv(gcL * Vm[P], Vm[D]);
+    const R aR2 = sizeof(R) == 4 ? gcR * Vp[P] * yDR : rdiv(gcR * Vp[P], Vp[D]);
     const bool roe = EXT == 1 && prm.riemann == 1;
     const bool marq = EXT == 2 && (prm.riemann == 5 || prm.riemann == 7);
     // hy_getFaceFlux.F90:364-383: the hybrid solver is HLL next to a marked cell, HLLC elsewhere
@@ -1085,7 +1157,7 @@ __device__ __forceinline__ int riemann(const DevParams &prm, int dir, const R *V
             } else if (SL < R(0) && qStar >= R(0)) {
                 const R numerL = SL - velNL, denomL = SL - qStar;
                 const R pStar = Vm[D] * numerL * (qStar - velNL) + Vm[P];
-                const R yd = rdiv(R(1), denomL);
+                const R yd = rcp_y(denomL);
                 const R dStar = rdiv_y(UL[0] * numerL, denomL, yd);
                 R UC[5];
                 UC[0] = dStar;
@@ -1099,7 +1171,7 @@ __device__ __forceinline__ int riemann(const DevParams &prm, int dir, const R *V
                 const R numerR = SR - velNR, denomR = SR - qStar;
                 const R numerL = SL - velNL;
                 const R pStar = Vm[D] * numerL * (qStar - velNL) + Vm[P];
-                const R yd = rdiv(R(1), denomR);
+                const R yd = rcp_y(denomR);
                 const R dStar = rdiv_y(UR[0] * numerR, denomR, yd);
                 R UC[5];
                 UC[0] = dStar;
@@ -1130,8 +1202,9 @@ __device__ __forceinline__ int riemann(const DevParams &prm, int dir, const R *V
     }
     // aux internal-energy and volume fluxes (hy_getFaceFlux.F90:444-453)
     if (OPT == OPT_DEFAULT || prm.use_aux_eint) {
-        if (F[0] > R(0)) { F[FVOL] = rdiv(F[0], Vm[D]); F[FEI] = F[0] * Vm[5]; }
-        else             { F[FVOL] = rdiv(F[0], Vp[D]); F[FEI] = F[0] * Vp[5]; }
+        const bool pos = F[0] > R(0);
+        F[FVOL] = sizeof(R) == 4 ? F[0] * (pos ? yDL : yDR) : rdiv(F[0], pos ? Vm[D] : Vp[D]);
+        F[FEI] = F[0] * (pos ? Vm[5] : Vp[5]);
     } else { F[FVOL] = R(0); F[FEI] = R(0); }
     return 0;
 }
