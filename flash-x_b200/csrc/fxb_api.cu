@@ -9,6 +9,7 @@
 
 #include <cuda_runtime.h>
 #include <cudaTypedefs.h>
+#include <stdint.h>
 #include <stdio.h>
 #include <stdlib.h>
 #include <string.h>
@@ -1132,9 +1133,43 @@ int lock_host_unk(const void *unk_host, size_t bytes)
     return FXB_OK;
 }
 
+// the interior rows (nxb cells x nunk slots) of every 3-D block from src to
+// dst, two blocked arrays of UNK's shape of which one is the caller's
+// page-locked memory, in elements of T (16 bytes where rows and pitches
+// allow it); wid: values per element
+template <class T>
+__global__ void __launch_bounds__(256) interior_rows_kernel(T *__restrict__ dst, const T *__restrict__ src, UnkGeom g,
+                                                            int nblk, int wid)
+{
+    const int row = g.nxb * g.nunk / wid;              // elements of a row's interior cells
+    const long pitch = (long)g.nig * g.nunk / wid;     // from one row of cells to the next
+    const long first = (long)g.ng * g.nunk / wid;      // before the first interior cell
+    const long per = (long)row * g.nyb * g.nzb, n = per * nblk;
+    const long step = (long)gridDim.x * blockDim.x;
+    for (long t0 = blockIdx.x * (long)blockDim.x + threadIdx.x; t0 < n; t0 += 4 * step) {
+        T v[4];
+        long at[4];
+#pragma unroll
+        for (int q = 0; q < 4; q++) {
+            const long t = t0 + q * step;
+            if (t >= n) break;
+            const long b = t / per, r = t - b * per, jk = r / row, e = r - jk * row, k = jk / g.nyb, j = jk - k * g.nyb;
+            at[q] = ((b * g.nkg + k + g.ng) * g.njg + j + g.ng) * pitch + first + e;
+            v[q] = __ldcs(src + at[q]);
+        }
+#pragma unroll
+        for (int q = 0; q < 4; q++)
+            if (t0 + q * step < n) __stcs(dst + at[q], v[q]);
+    }
+}
+
 // the interior rows of every block, between the caller's UNK and the device
-// mirror: one 3-D copy over all blocks in 2-D (their rows are evenly
-// spaced), one per block in 3-D (the k guard planes separate the blocks)
+// mirror.  2-D: one strided copy over all blocks (their rows are evenly
+// spaced).  3-D: the k guard planes separate the blocks, so the copy engine
+// would need a copy per block, 6 us of host time each (2,805 blocks of 8^3,
+// 126 MB: 17 ms each way against 2.5 ms of bus time); one kernel reads or
+// writes the page-locked memory instead.  Memory that the device cannot
+// address keeps the copies.
 int copy_interior_rows(double *dst, const double *src, cudaMemcpyKind kind)
 {
     const UnkGeom g = unk_geom();
@@ -1150,6 +1185,22 @@ int copy_interior_rows(double *dst, const double *src, cudaMemcpyKind kind)
         CK(cudaMemcpy3DAsync(&p, L.stream));
         return FXB_OK;
     }
+    const bool in = kind == cudaMemcpyHostToDevice;
+    void *host = nullptr;
+    if (cudaHostGetDevicePointer(&host, in ? const_cast<double *>(src) : dst, 0) == cudaSuccess && host) {
+        double *kd = in ? dst : (double *)host;
+        const double *ks = in ? (const double *)host : src;
+        // 16-byte elements where rows, pitches and the guard cells before a row are whole pairs of values
+        const bool wide = g.ng * g.nunk % 2 == 0 && g.nxb * g.nunk % 2 == 0 && g.nig * g.nunk % 2 == 0 &&
+                          ((uintptr_t)host & 15) == 0;
+        if (wide)
+            interior_rows_kernel<double2><<<148 * 8, 256, 0, L.stream>>>((double2 *)kd, (const double2 *)ks, g, L.nblk, 2);
+        else
+            interior_rows_kernel<double><<<148 * 8, 256, 0, L.stream>>>(kd, ks, g, L.nblk, 1);
+        CK(cudaGetLastError());
+        return FXB_OK;
+    }
+    cudaGetLastError();
     p.extent = make_cudaExtent(w, g.nyb, g.nzb);
     for (int b = 0; b < L.nblk; b++) {
         p.srcPos = p.dstPos = make_cudaPos(x0, g.ng, (size_t)b * g.nkg + g.ng);
