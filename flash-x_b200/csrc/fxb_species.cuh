@@ -41,7 +41,8 @@ struct SpecArgs {
     double dt_arg;
     const double *dtv;
     DevParams prm;
-    const void *fd[3];               // mass flux of every face of direction d (Grid3::fidx), type R
+    const void *fd[3];               // mass flux of every face of direction d (Grid3::fidx; 3-D: slot 0 of the
+                                     // tiled flux array), type R
     const void *flat;                // flattening coefficients of the hydro step (padded box), type R
     const unsigned char *ctufb[3];   // 3-D: CTU fallback of each face-state cell (Grid3::widx)
     void *sg;                        // [3][ns][npad] of R
@@ -253,7 +254,8 @@ __global__ void __launch_bounds__(256) spec_update_kernel(const SpecArgs a)
                 const R *f = (const R *)a.fd[d];
                 const R *L = sl + ((long)d * a.ns + n) * a.nwmax, *Rr = sr + ((long)d * a.ns + n) * a.nwmax;
                 // face between cell c - e_d and c, and between c and c + e_d
-                const double fl = (double)f[G.fidx(d, i, j, k)], fr = (double)f[G.fidx(d, i + di, j + dj, k + dk)];
+                const long il = G.fidx(d, i, j, k), ir = G.fidx(d, i + di, j + dj, k + dk);
+                const double fl = (double)f[a.ndim == 3 ? tile_at<NF>(il) : il], fr = (double)f[a.ndim == 3 ? tile_at<NF>(ir) : ir];
                 FL[d] = fl < 0. ? fl * (double)L[G.widx(d, i, j, k)] : fl * (double)Rr[G.widx(d, i - di, j - dj, k - dk)];
                 FR[d] = fr < 0. ? fr * (double)L[G.widx(d, i + di, j + dj, k + dk)] : fr * (double)Rr[G.widx(d, i, j, k)];
             }

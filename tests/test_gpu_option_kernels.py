@@ -10,6 +10,7 @@ import dataclasses
 import numpy as np
 import pytest
 
+from flashx_b200 import amr as A
 from flashx_b200 import simulations as S
 from flashx_b200.hydro import HydroDevice
 from flashx_b200.params import (BC_OUTFLOW, BC_PERIODIC, BC_REFLECTING, DENS, EINT, ENER, GAMC, GAME,
@@ -71,3 +72,77 @@ def test_2d_option_matches_oracle(oracle, need_gpu, name):
     geom = Geometry(2, 16, 16, 1, 3, 2, 1, bc=(BC_REFLECTING, BC_OUTFLOW, BC_PERIODIC, BC_PERIODIC) + (BC_OUTFLOW,) * 2)
     hp = dataclasses.replace(HydroParams(gamma=5.0 / 3.0), **OPTIONS[name])
     _check(*_steps(oracle, geom, hp, S.noisy_gas(geom, hp)))
+
+
+OPTIONS_3D = dict(OPTIONS, no_ctu={"use_3dFullCTU": False}, pressure_source={"hy_fPresInMomFlux": 0.5},
+                  gravity={"useGravity": True, "gravity": (0.02, -0.03, -0.1)},
+                  weno_gravity={"order": 5, "useGravity": True, "gravity": (0.02, -0.03, -0.1)})
+
+
+@pytest.mark.parametrize("name", sorted(OPTIONS_3D))
+def test_3d_option_matches_oracle(oracle, need_gpu, name):
+    geom = Geometry(3, 8, 8, 8, 3, 2, 1,
+                    bc=(BC_REFLECTING, BC_OUTFLOW, BC_PERIODIC, BC_PERIODIC, BC_REFLECTING, BC_REFLECTING))
+    hp = dataclasses.replace(HydroParams(gamma=5.0 / 3.0), **OPTIONS_3D[name])
+    _check(*_steps(oracle, geom, hp, S.noisy_gas(geom, hp)))
+
+
+# extents where the sweeps' tiles and segments end unevenly: odd ones, the
+# fewest cells a block can have, and one long axis at a time (several x
+# segments, line segments and planes per CTA)
+@pytest.mark.parametrize("order", [3, 5])
+@pytest.mark.parametrize("shape", [((5, 6, 7), (2, 1, 3)), ((4, 4, 4), (1, 1, 1)), ((16, 4, 4), (11, 1, 1)),
+                                   ((4, 16, 4), (1, 11, 1)), ((4, 4, 16), (1, 1, 11)), ((33, 9, 4), (1, 1, 1))])
+def test_3d_sweep_extents_match_oracle(oracle, need_gpu, shape, order):
+    (nx, ny, nz), (bx, by, bz) = shape
+    for bc in ((BC_PERIODIC,) * 6, (BC_OUTFLOW,) * 2 + (BC_REFLECTING,) * 2 + (BC_PERIODIC,) * 2,
+               (BC_REFLECTING,) * 2 + (BC_PERIODIC,) * 2 + (BC_OUTFLOW,) * 2):
+        geom = Geometry(3, nx, ny, nz, bx, by, bz, bc=bc,
+                        bbox=((0.0, float(nx * bx)), (0.0, float(ny * by)), (0.0, float(nz * bz))))
+        hp = HydroParams(gamma=5.0 / 3.0, order=order)
+        _check(*_steps(oracle, geom, hp, S.noisy_gas(geom, hp)))
+
+
+@pytest.mark.parametrize("name", ["default", "vanLeer", "weno", "HLL"])
+def test_amr_option_matches_oracle(oracle, need_gpu, name):
+    geom = Geometry(3, 8, 8, 8, 2, 2, 2, bc=(BC_PERIODIC,) * 4 + (BC_REFLECTING,) * 2)
+    hp = dataclasses.replace(HydroParams(), **OPTIONS[name])
+    mesh, unk = A.levelset_problem(geom, hp, 2)
+    am = oracle.Amr(oracle.make_params(geom.as_dict(), hp), mesh.levels, mesh.bcoords)
+    dt = 0.4 * am.compute_dt(unk)
+    ref = unk.copy()
+    for _ in range(2):
+        am.hydro_step(ref, dt)
+    g = geom.nguard
+    out = {}
+    for prec in ("fp64", "mixed"):
+        dev = HydroDevice(geom, hp, prec, mesh=mesh)
+        dev.attach_unk(unk.copy())
+        for i in range(2):
+            dev.Hydro(i * dt, dt, dt)
+        o = unk.copy()
+        dev.sync_to_host(o)
+        dev.close()
+        out[prec] = o[:, g:-g, g:-g, g:-g][..., HYDRO_VARS]
+    _check(out, ref[:, g:-g, g:-g, g:-g][..., HYDRO_VARS])
+
+
+# rows of whole 16-byte pairs, and (odd block sizes, odd slot counts) not
+@pytest.mark.parametrize("n", [8, 5])
+def test_3d_interior_transfers_move_every_row(need_gpu, n):
+    geom = Geometry(3, n, n + 1, n + 2, 3, 2, 2, bc=(BC_PERIODIC,) * 6)
+    hp = HydroParams()
+    unk = S.noisy_gas(geom, hp)
+    dev = HydroDevice(geom, hp, "fp64")
+    dev.attach_unk(unk.copy())
+    other = unk.copy()
+    other[..., DENS] *= 2.0
+    dev.put_interior(other)
+    got = np.full(geom.unk_shape, -7.0)
+    dev.get_interior(got)
+    g = geom.nguard
+    inner = np.s_[:, g:-g, g:-g, g:-g]
+    assert np.array_equal(got[inner][..., HYDRO_VARS], other[inner][..., HYDRO_VARS])
+    got[inner] = -7.0
+    assert np.all(got == -7.0), "guard cells keep their values"
+    dev.close()
