@@ -19,9 +19,10 @@
 //      with the boundary conditions resolved by map_axis)
 //   B  x: eigensystem + limited slopes of cells i=-2..17, j=0..15      -> s.DB
 //   C  x: PPM/WENO face states of i=-1..16, j=0..15, minus dt/2dy*sig_y -> s.W
-//   D  x: HLLC/HLL on faces i=0..16                                     -> s.F
-//   E  owner threads: x part of the conserved and aux-eint update (registers)
-//   F..H the same for y
+//   D  x: HLLC/HLL on faces i=0..16 -> s.F; y slopes                    -> s.DB
+//   E  owner threads: x part of the conserved and aux-eint update (registers);
+//      y face states -> s.W
+//   H  y faces                                                          -> s.F
 //   I  owner threads: y update, energyFix, Eos, store, CFL rate max
 #pragma once
 #include "fxb_device.cuh"
@@ -90,7 +91,8 @@ constexpr int NOWN = T2 * T2;      // owner cells of a tile
 
 template <class R> struct Smem2D {
     R V[8][WIN][WP];
-    R DBF[NF * NFC];               // slopes [6][NDB], then fluxes [8][NFC]
+    R DB[6 * NDB];                 // slopes [6][NDB]
+    R F[NF * NFC];                 // fluxes [8][NFC]
     R SG[6][KeepSig<R>::value ? NDB : 1];   // sigma of the other direction at the slope cells (global order)
     R W[12][NW];                   // Wp (D,VX,VY,VZ,P,EI), then Wm
     R EB[4][EBW * EBW];            // eigensystem base: cf, ahinv, lp, a2inv (eb_at)
@@ -179,7 +181,7 @@ __device__ __forceinline__ void analysis_stage(const Args2D &a, Smem2D<R> &s, in
         eigen_dir(eb, c[1], e);
         tvd_slope<R, OPT>(a.prm, e, Vm, c, Vp, db);
 #pragma unroll
-        for (int k = 0; k < 6; k++) s.DBF[k * NDB + t] = db[k];
+        for (int k = 0; k < 6; k++) s.DB[k * NDB + t] = db[k];
     }
     if (KeepSig<R>::value) {
         R sg[6];
@@ -260,9 +262,9 @@ __device__ __forceinline__ void states_stage(const Args2D &a, Smem2D<R> &s, int 
         R dbN[6], db0[6], dbP[6];
 #pragma unroll
         for (int k = 0; k < 6; k++) {
-            dbN[k] = s.DBF[k * NDB + dbi - dbstep];
-            db0[k] = s.DBF[k * NDB + dbi];
-            dbP[k] = s.DBF[k * NDB + dbi + dbstep];
+            dbN[k] = s.DB[k * NDB + dbi - dbstep];
+            db0[k] = s.DB[k * NDB + dbi];
+            dbP[k] = s.DB[k * NDB + dbi + dbstep];
         }
         ppm_interfaces(Vm, Vc, Vp, dbN, db0, dbP, vecL, vecR);
         if (EXT && a.prm.steepening)
@@ -354,7 +356,7 @@ __device__ __forceinline__ void faces_stage(const Args2D &a, Smem2D<R> &s, int d
         eint_fluxes(a.prm, VL, VR, F);
     }
 #pragma unroll
-    for (int k = 0; k < NF; k++) s.DBF[k * NFC + t] = F[k];
+    for (int k = 0; k < NF; k++) s.F[k * NFC + t] = F[k];
 }
 
 // dynamic shared memory of one CTA: the stages' arrays plus 128 bytes to
@@ -366,7 +368,7 @@ constexpr unsigned kWinBoxBytes = 8u * WIN * WP * 8u;
 // face states and eigensystem bases (unused during stage A), which follows
 // the window at a 128-byte aligned offset
 static_assert(sizeof(float) * 8 * WIN * WP % 128 == 0, "FP32 window size keeps the staging area aligned");
-static_assert(sizeof(float) * (NF * NFC + 6 * NDB + 12 * NW + 4 * EBW * EBW) >= kWinBoxBytes,
+static_assert(sizeof(float) * (6 * NDB + NF * NFC + 6 * NDB + 12 * NW + 4 * EBW * EBW) >= kWinBoxBytes,
               "FP32 staging area holds the FP64 window box");
 
 // ORDER: the reconstruction order, 0 where it is read at run time (extended
@@ -397,7 +399,7 @@ hydro2d_kernel(const __grid_constant__ Args2D a)
     bool ok = true;
     if (tma) {
         double *stage = sizeof(R) == 8 ? reinterpret_cast<double *>(&s.V[0][0][0])
-                                       : reinterpret_cast<double *>(&s.DBF[0]);
+                                       : reinterpret_cast<double *>(&s.DB[0]);
         if (tid == 0) mbar_init(&wbar, 1);
         __syncthreads();
         if (tid == 0) {
@@ -500,17 +502,27 @@ hydro2d_kernel(const __grid_constant__ Args2D a)
                                   order);
     }
     __syncthreads();
-    // ---- D: x faces
+    // ---- D: x faces; with them the y slopes and sigma_x, which need the window
+    // only, and the owners' mean x face pressure, before y overwrites the states
+    for (int t = tid; t < NDB; t += NT2) {
+        int ii = t % T2, jj = t / T2 - 2;
+        analysis_stage<R, OPT>(a, s, 1, t, ii + 3, jj + 3, ppm);
+    }
     for (int t = tid; t < NFC; t += NT2) {
         int fi = t % (T2 + 1), jj = t / (T2 + 1);
         faces_stage<R, EXT, OPT>(a, s, 0, t, jj * (T2 + 2) + fi, jj * (T2 + 2) + fi + 1, fi + 2, jj + 3, fi + 3, jj + 3);
         if (EXT && a.fd[0] && (fi < T2 || tx0 + T2 == a.nx))   // the species' mass fluxes
-            ((R *)a.fd[0])[(long)(ty0 + jj) * (a.nx + 1) + tx0 + fi] = s.DBF[FD * NFC + t];
+            ((R *)a.fd[0])[(long)(ty0 + jj) * (a.nx + 1) + tx0 + fi] = s.F[FD * NFC + t];
+    }
+    double pav = 0.;
+    if (owner) {
+        int w = oj * (T2 + 2) + oi + 1;
+        pav = 0.5 * ((double)s.W[6 + P][w] + (double)s.W[P][w]);
     }
     __syncthreads();
 
     // ---- E: owner threads, x part of the update
-    double U0[5], dens0 = 0., Ax = 0., Bx = 0., pav = 0., SphX = 0., eint0 = 0.;
+    double U0[5], dens0 = 0., Ax = 0., Bx = 0., SphX = 0., eint0 = 0.;
     const double dtdx = dt_dx, dtdy = dt_dy;
     if (owner) {
         double vx, vy, vz, en = s.OWN[0][tid];
@@ -527,21 +539,12 @@ hydro2d_kernel(const __grid_constant__ Args2D a)
         int fl = oj * (T2 + 1) + oi, fr = fl + 1;
 #pragma unroll
         for (int v = 0; v < 5; v++)
-            U0[v] = U0[v] - dtdx * ((double)s.DBF[v * NFC + fr] - (double)s.DBF[v * NFC + fl]);
-        Ax = (double)s.DBF[FEI * NFC + fl] - (double)s.DBF[FEI * NFC + fr];
-        Bx = (double)s.DBF[FVOL * NFC + fl] - (double)s.DBF[FVOL * NFC + fr];
-        SphX = ((double)s.DBF[FP * NFC + fl] - (double)s.DBF[FP * NFC + fr]) * (1.0 - a.prm.fpres) / a.dx;
-        int w = oj * (T2 + 2) + oi + 1;
-        pav = 0.5 * ((double)s.W[6 + P][w] + (double)s.W[P][w]);
+            U0[v] = U0[v] - dtdx * ((double)s.F[v * NFC + fr] - (double)s.F[v * NFC + fl]);
+        Ax = (double)s.F[FEI * NFC + fl] - (double)s.F[FEI * NFC + fr];
+        Bx = (double)s.F[FVOL * NFC + fl] - (double)s.F[FVOL * NFC + fr];
+        SphX = ((double)s.F[FP * NFC + fl] - (double)s.F[FP * NFC + fr]) * (1.0 - a.prm.fpres) / a.dx;
     }
-    __syncthreads();
 
-    // ---- F: y slopes and sigma_x
-    for (int t = tid; t < NDB; t += NT2) {
-        int ii = t % T2, jj = t / T2 - 2;
-        analysis_stage<R, OPT>(a, s, 1, t, ii + 3, jj + 3, ppm);
-    }
-    __syncthreads();
     // ---- G: y face states
     for (int t = tid; t < NW; t += NT2) {
         int ii = t % T2, jj = t / T2 - 1;
@@ -554,7 +557,7 @@ hydro2d_kernel(const __grid_constant__ Args2D a)
         int ii = t % T2, fj = t / T2;
         faces_stage<R, EXT, OPT>(a, s, 1, t, fj * T2 + ii, (fj + 1) * T2 + ii, ii + 3, fj + 2, ii + 3, fj + 3);
         if (EXT && a.fd[1] && (fj < T2 || ty0 + T2 == a.ny))
-            ((R *)a.fd[1])[(long)(ty0 + fj) * a.nx + tx0 + ii] = s.DBF[FD * NFC + t];
+            ((R *)a.fd[1])[(long)(ty0 + fj) * a.nx + tx0 + ii] = s.F[FD * NFC + t];
     }
     __syncthreads();
 
@@ -565,10 +568,10 @@ hydro2d_kernel(const __grid_constant__ Args2D a)
         int fl = oj * T2 + oi, fr = fl + T2;
 #pragma unroll
         for (int v = 0; v < 5; v++)
-            U0[v] = U0[v] - dtdy * ((double)s.DBF[v * NFC + fr] - (double)s.DBF[v * NFC + fl]);
-        double Ay = (double)s.DBF[FEI * NFC + fl] - (double)s.DBF[FEI * NFC + fr];
-        double By = (double)s.DBF[FVOL * NFC + fl] - (double)s.DBF[FVOL * NFC + fr];
-        double SphY = ((double)s.DBF[FP * NFC + fl] - (double)s.DBF[FP * NFC + fr]) * (1.0 - prm.fpres) / a.dy;
+            U0[v] = U0[v] - dtdy * ((double)s.F[v * NFC + fr] - (double)s.F[v * NFC + fl]);
+        double Ay = (double)s.F[FEI * NFC + fl] - (double)s.F[FEI * NFC + fr];
+        double By = (double)s.F[FVOL * NFC + fl] - (double)s.F[FVOL * NFC + fr];
+        double SphY = ((double)s.F[FP * NFC + fl] - (double)s.F[FP * NFC + fr]) * (1.0 - prm.fpres) / a.dy;
         int w = (oj + 1) * T2 + oi;
         pav = pav * 0.5 + ((double)s.W[6 + P][w] + (double)s.W[P][w]) * 0.25;
         double inten = 0.;
