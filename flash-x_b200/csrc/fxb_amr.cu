@@ -844,6 +844,8 @@ Args3D batch_args(const double *dtv, double dt)
     a.dxl = S.d_dxl;
     for (int q = 0; q < 4; q++) a.cta[q] = S.cta[q];
     a.odata = S.store[1 - S.cur]; a.o_vstride = S.vstride; a.o_bstride = S.bstride;
+    a.bflux = S.bflux;
+    a.nfc = S.nfc;
     const size_t r = rsize();
     a.sig_bstride = (long)(sig3d_bytes(S.n, S.n, S.n, r) / r);
     a.slp_bstride = (long)(slp3d_bytes(S.n, S.n, S.n, r) / r);
@@ -1384,7 +1386,10 @@ int batched_step(const double *dtv, double dt, int &nl)
         if (mixed) launch_amr3d_fluxes_mixed(a, cnt, all, S.C.stream);
         else launch_amr3d_fluxes_fp64(a, cnt, all, S.C.stream);
     };
+    // the default options' sweeps store the boundary fluxes themselves
+    const bool ext = extended_options(S.C.dprm);
     auto emit = [&](int cnt) {
+        if (!ext) return;
         if (mixed) launch_amr3d_emit_mixed(a, cnt, S.bflux, S.nfc, S.C.stream);
         else launch_amr3d_emit_fp64(a, cnt, S.bflux, S.nfc, S.C.stream);
     };
@@ -1396,21 +1401,21 @@ int batched_step(const double *dtv, double dt, int &nl)
         if (mixed) launch_amr3d_update_mixed(a, cnt, S.C.stream); else launch_amr3d_update_fp64(a, cnt, S.C.stream);
     };
     // sigma (+ flattening), then per direction the slopes, face states and
-    // fluxes (one fused kernel in FP32; slopes (PPM), face states and fluxes
-    // as separate kernels in FP64)
-    const int pipe = 1 + (S.C.prm.flattening ? 1 : 0) + 3 * (mixed ? 1 : (S.C.prm.order == 3 ? 3 : 2));
+    // fluxes (one kernel; with extended options in FP64 slopes (PPM), face
+    // states and fluxes as separate kernels)
+    const int pipe = 1 + (S.C.prm.flattening ? 1 : 0) + 3 * (mixed || !ext ? 1 : (S.C.prm.order == 3 ? 3 : 2));
     if (S.nstep <= S.batch) {
         a.batch = S.d_step_entries;
         nl += fill_batch(a.batch, S.nstep, S.cur);
         fluxes(S.nstep); emit(S.nstep); correct(S.nstep); update(S.nstep);
-        nl += pipe + 3;
+        nl += pipe + 2 + ext;
     } else {
         for (int l0 = 0; l0 < S.nstep; l0 += S.batch) {
             int cnt = std::min(S.batch, S.nstep - l0);
             a.batch = S.d_step_entries + S.nstep + l0;
             nl += fill_batch(a.batch, cnt, S.cur);
             fluxes(cnt); emit(cnt); update(cnt);
-            nl += pipe + 2;
+            nl += pipe + 1 + ext;
         }
         for (int l0 = 0; l0 < S.nstep_finer; l0 += S.batch) {
             int cnt = std::min(S.batch, S.nstep_finer - l0);

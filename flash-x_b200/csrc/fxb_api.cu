@@ -564,11 +564,11 @@ int launch_species(int src, const double *dtv, double dt)
 }
 
 // kernels of one 3-D step: sigma, per direction the slopes, face states and
-// fluxes (one fused kernel in FP32; slopes (PPM), face states and fluxes as
-// separate kernels in FP64), the update
+// fluxes (one kernel; with extended options in FP64 slopes (PPM), face states
+// and fluxes as separate kernels), the update
 int hydro3d_launches(const fxb_params &p)
 {
-    const int per_dir = p.precision == FXB_MIXED ? 1 : (p.order == 3 ? 3 : 2);
+    const int per_dir = p.precision == FXB_MIXED || !extended_options(L.dprm) ? 1 : (p.order == 3 ? 3 : 2);
     return 1 + 3 * per_dir + 1;
 }
 // launches of one uniform-grid step (flattening and species add kernels)
@@ -990,7 +990,8 @@ static int ug_tune()
                  "staging: %s (ms per step: TMA %.3f, per-thread loads %.3f%s)", L.use_tma ? "TMA" : "per-thread loads",
                  t[1], t[0], off ? ", tuning off" : "");
     } else {
-        const bool fused = L.prm.precision == FXB_MIXED;
+        // the default options' sweeps choose their own grids
+        const bool fused = L.prm.precision == FXB_MIXED, ext = extended_options(L.dprm);
         float cur = base;
         // FXB_UG_CTA="s,f,x,u" and FXB_UG_T1="x,y,z" fix the shapes instead
         const char *ec = getenv("FXB_UG_CTA"), *et = getenv("FXB_UG_T1");
@@ -1009,7 +1010,7 @@ static int ug_tune()
         if (!off && !ec && !et) {
             const int cand[4] = {2, 4, 8, 16};
             for (int q = 0; q < 4; q++) {
-                if (fused && (q == 1 || q == 2)) continue;     // the fused kernel's grid follows its tiles
+                if ((fused || !ext) && (q == 1 || q == 2)) continue;     // the fused kernel's grid follows its tiles
                 int keep = L.ug_cta[q];
                 for (int c : cand) {
                     if (c == keep) continue;
@@ -1021,7 +1022,7 @@ static int ug_tune()
                     L.ug_cta[q] = keep;
                 }
             }
-            if (fused)
+            if (fused && ext)
                 for (int d = 0; d < 3; d++) {
                     int keep = L.sf_t1[d];
                     for (int t1 : {1, 2, 4, 8, 16}) {

@@ -90,6 +90,8 @@ struct Args3D {
     void *divu = nullptr;       // AMR: DivU scratch per batch entry, box [-3, n+2]^3 of R
     long divu_bstride = 0;
     long rate_c0 = 0, rate_c1 = 0x7fffffffffffffffL;   // cells [c0, c1) enter the CFL rate (a slab's own)
+    void *bflux = nullptr;      // AMR: boundary fluxes [leaf][face][slot][nfc], stored by the default-option sweeps
+    long nfc = 0;
     unsigned char *ctufb[3] = {nullptr, nullptr, nullptr};   // species on: 1 where the CTU fallback fired (Grid3::widx)
     const unsigned char *shok = nullptr;   // shock detector on (uniform grid): the flag of every cell
 };
@@ -454,8 +456,10 @@ __device__ __forceinline__ void sig3d_kernel_body(const Args3D &a, const VB vb)
         }
     }
 }
+// FP32 on the uniform grid: four CTAs per SM (64 registers), 83 instead of
+// 97 us at 128^3; FP64 three (80), with four it spills (163 instead of 110 us)
 template <class R, bool AMR>
-__global__ void __launch_bounds__(256) sig3d_kernel(const Args3D a)
+__global__ void __launch_bounds__(256, sizeof(R) == 4 ? 4 : 3) sig3d_kernel(const Args3D a)
 {
     sig3d_kernel_body<R, AMR>(a, hw_block());
 }
@@ -1002,9 +1006,6 @@ __device__ __forceinline__ void update3d_kernel_body(const Args3D &a, const VB v
     __syncthreads();
     double *out = AMR ? a.odata + (long)X.m.out_blk * a.o_bstride : a.out;
     const long ovs = AMR ? a.o_vstride : a.vstride;
-    // the face-pressure source has the factor 1 - hy_fPresInMomFlux: with the
-    // default 1 the pressure slot is not read, and its zero is formed from the
-    // momentum fluxes, which are not finite where the pressure is not
     const bool fp = prm.fpres != 1.0;
     double rate = 0.;
     FXB_VB_LOOP(c, n, vb) {
@@ -1016,45 +1017,49 @@ __device__ __forceinline__ void update3d_kernel_body(const Args3D &a, const VB v
         double dens0 = in[D * vs];
         double vx0 = in[VX * vs], vy0 = in[VY * vs], vz0 = in[VZ * vs];
         double en0 = in[DV_ENER * vs], eint0 = in[EI * vs];
-        double U0[5] = {dens0, vx0 * dens0, vy0 * dens0, vz0 * dens0, dens0 * en0};
-        double Sph[3];
-        double A[3], B[3], pav = 0.;
+        // the mean of the six face pressures first: with it every direction's
+        // fluxes are used as they arrive and none stays in registers
+        double pav = 0.;
 #pragma unroll
         for (int d = 0; d < 3; d++) {
-            const R *w = X.wst[d];
+            const R *w = X.wst[d] + G.widx(d, i, j, k);
             const long nw = G.nw(d);
+            const double sum = (double)w[(long)a.pw_wm[d] * nw] + (double)w[(long)a.pw_wp[d] * nw];
+            if (d == 0) pav = 0.5 * sum;
+            else if (d == 1) pav = pav * 0.5 + sum * 0.25;
+            else pav = divk<6>(pav * 4.0 + sum);
+        }
+        double U0[5] = {dens0, vx0 * dens0, vy0 * dens0, vz0 * dens0, dens0 * en0};
+        double inten = dens0 * eint0;
+#pragma unroll
+        for (int d = 0; d < 3; d++) {
             const long s1 = d == 0 ? 1 : d == 1 ? a.nx : (long)a.nx * a.ny;   // the next face along d
             const long f0 = G.fidx(d, i, j, k);
             const R *fl = X.flx[d] + tile_at<NF>(f0), *fr = X.flx[d] + tile_at<NF>(f0 + s1);
             const double dtdl = uq[d];
 #pragma unroll
-            for (int v = 0; v < 5; v++) {
-                const double l = (double)fl[v * TILE3], r = (double)fr[v * TILE3];
-                U0[v] = U0[v] - dtdl * (r - l);
-                if (v == FMX + d && !fp) Sph[d] = (l - r) * 0.0;
-            }
-            A[d] = (double)fl[FEI * TILE3] - (double)fr[FEI * TILE3];
-            B[d] = (double)fl[FVOL * TILE3] - (double)fr[FVOL * TILE3];
-            if (fp) {
-                const double del = d == 0 ? X.dx : d == 1 ? X.dy : X.dz;
-                Sph[d] = ((double)fl[FP * TILE3] - (double)fr[FP * TILE3]) * (1.0 - prm.fpres) / del;
-            }
-            const long wc = G.widx(d, i, j, k);
-            const double sum = (double)w[(long)a.pw_wm[d] * nw + wc] + (double)w[(long)a.pw_wp[d] * nw + wc];
-            if (d == 0) pav = 0.5 * sum;
-            else if (d == 1) pav = pav * 0.5 + sum * 0.25;
-            else pav = divk<6>(pav * 4.0 + sum);
+            for (int v = 0; v < 5; v++) U0[v] = U0[v] - dtdl * ((double)fr[v * TILE3] - (double)fl[v * TILE3]);
+            const double A = (double)fl[FEI * TILE3] - (double)fr[FEI * TILE3];
+            const double B = (double)fl[FVOL * TILE3] - (double)fr[FVOL * TILE3];
+            inten = inten + dtdl * (A + pav * B);
         }
-        double inten = 0.;
-        if (prm.use_aux_eint) {
-            inten = dens0 * eint0;
-#pragma unroll
-            for (int d = 0; d < 3; d++) inten = inten + uq[d] * (A[d] + pav * B[d]);
-            inten = inten + dt * 0.0;
-        }
+        inten = inten + dt * 0.0;
+        // the face-pressure source of direction d has the factor 1 -
+        // hy_fPresInMomFlux: with the default 1 the pressure slot is not read
+        // and the source is zero, or not a number where the momentum is not
+        // finite (as the momentum flux is where the pressure is not)
         U0[0] = U0[0] + dt * 0.;
 #pragma unroll
-        for (int d = 0; d < 3; d++) U0[1 + d] = U0[1 + d] + dt * (0. + Sph[d]);
+        for (int d = 0; d < 3; d++) {
+            double Sph = U0[1 + d] * 0.0;
+            if (fp) {
+                const long s1 = d == 0 ? 1 : d == 1 ? a.nx : (long)a.nx * a.ny;
+                const long f0 = G.fidx(d, i, j, k);
+                Sph = ((double)X.flx[d][tile_at<NF>(f0) + FP * TILE3] - (double)X.flx[d][tile_at<NF>(f0 + s1) + FP * TILE3]) *
+                      (1.0 - prm.fpres) / (d == 0 ? X.dx : d == 1 ? X.dy : X.dz);
+            }
+            U0[1 + d] = U0[1 + d] + dt * (0. + Sph);
+        }
         U0[4] = U0[4] + dt * 0.;
         if (prm.use_gravity) {
             const double momOld[3] = {vx0 * dens0, vy0 * dens0, vz0 * dens0};

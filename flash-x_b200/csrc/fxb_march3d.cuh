@@ -121,6 +121,28 @@ __device__ __forceinline__ void sweep_states(const Args3D &a, const Ctx3<R, AMR>
     }
 }
 
+// the fluxes of a face of direction DIR into the flux array; on an AMR leaf
+// also into its boundary fluxes (Grid_putFluxData) when the face is on the
+// block's boundary (c = 0 or N; t1, t2: the face's transverse cell).  The
+// pressure slot only where the update reads it (fp).
+template <class R, bool AMR, int DIR>
+__device__ __forceinline__ void store_fluxes(const Args3D &a, const Ctx3<R, AMR> &X, int i, int j, int k, bool fp,
+                                             const R F[NF])
+{
+    R *f = X.flx[DIR] + tile_at<NF>(X.G.fidx(DIR, i, j, k));
+#pragma unroll
+    for (int q = 0; q < NF; q++) if (q != FP || fp) f[q * TILE3] = F[q];
+    if constexpr (AMR) {
+        const int c = DIR == 0 ? i : DIR == 1 ? j : k, N = DIR == 0 ? a.nx : DIR == 1 ? a.ny : a.nz;
+        if (c == 0 || c == N) {
+            const int t1 = DIR == 0 ? j : i, t2 = DIR == 2 ? j : k, n1 = DIR == 0 ? a.ny : a.nx;
+            R *b = (R *)a.bflux + ((long)X.m.leaf * 6 + 2 * DIR + (c == N)) * NF * a.nfc + t2 * n1 + t1;
+#pragma unroll
+            for (int q = 0; q < NF; q++) if (q != FP || fp) b[q * a.nfc] = F[q];
+        }
+    }
+}
+
 constexpr int MARCH_T = 128;          // threads per CTA
 // resident CTAs per SM: 168 registers per thread in FP64 (shared memory allows
 // no fourth CTA), 96 in FP32 (six CTAs of 80 registers: PPM 128^3 0.66 instead
@@ -266,9 +288,7 @@ __global__ void __launch_bounds__(MARCH_T, MarchMinB<R>::value) march3d_kernel(c
             get(SL::wp, VL);
             const int er = riemann<R, 0, OPT>(a.prm, DIR, VL, gcl, gel, Wm, gc, ge, F);
             if (er) atomicOr(a.err, er);
-            R *f = X.flx[DIR] + tile_at<NF>(DIR == 1 ? G.fidx(1, i, c - 1, t2) : G.fidx(2, i, t2, c - 1));
-#pragma unroll
-            for (int q = 0; q < NF; q++) if (q != FP || fp) f[q * TILE3] = F[q];
+            store_fluxes<R, AMR, DIR>(a, X, i, DIR == 1 ? c - 1 : t2, DIR == 1 ? t2 : c - 1, fp, F);
         }
         if (c == f1) break;
         if (c > c0) put(SL::wp, Wp);               // of cell c - 1
@@ -396,6 +416,9 @@ __global__ void __launch_bounds__(SWX_T, SwxMinB<R>::value) sweepx3d_kernel(cons
     // this thread's sigmas: sigma_y of the planes k - 1, k, k + 1 (six values
     // each, in turn), then sigma_z of plane k
     R *const sS = sW + 6 * SWX_T + threadIdx.x;
+    // sigma_z of plane k of the lines before the tile's first and behind its
+    // last one, [6][two lines of Lt cells in rows of SWX_T]
+    R *const sH = sW + 30 * SWX_T;
     if (t < 5)
         sq[t] = t == 0 ? dt / X.dx
                 : t == 1 ? 0.5 * dt / X.dx
@@ -453,10 +476,23 @@ __global__ void __launch_bounds__(SWX_T, SwxMinB<R>::value) sweepx3d_kernel(cons
         for (int v = 0; v < 6; v++) cp_async(sS + (slot + v) * SWX_T, p + v * TILE3);
     };
     int rm = 0, rc = 6, rp = 12;       // slots of sigma_y of the planes k - 1, k, k + 1
+    // sigma_z beside this line: the neighbour thread's own, or the outer lines'
+    const bool first = l1 == 0, last = l1 + 1 == T1 || j + 1 == N1;
+    const R *const hm = first ? sH + ld : sS - Lt + 18 * SWX_T, *const hp = last ? sH + Lt + ld : sS + Lt + 18 * SWX_T;
+    auto copy_sigz = [&](int k) {
+        copy_sig(18, 2, k);
+#pragma unroll
+        for (int side = 0; side < 2; side++) {
+            if (side ? !last : !first) continue;
+            const R *p = sweep_sig_at<0>((const R *)X.sig, G, 2 + side, c, j, k);
+#pragma unroll
+            for (int v = 0; v < 6; v++) cp_async(sH + v * SWX_T + side * Lt + ld, p + v * TILE3);
+        }
+    };
     copy_plane(k0, 0);
     if (AHEAD && st) {
         copy_sig(rm, 1, k0 - 1); copy_sig(rc, 1, k0); copy_sig(rp, 1, k0 + 1);
-        copy_sig(18, 2, k0);
+        copy_sigz(k0);
         cp_async_commit();
     }
     for (int k = k0; k < k1; k++) {
@@ -503,21 +539,12 @@ __global__ void __launch_bounds__(SWX_T, SwxMinB<R>::value) sweepx3d_kernel(cons
 #pragma unroll
                 for (int v = 0; v < 12; v++) own[v] = __ldg(gp[v / 6] + v % 6 * TILE3);
             }
-            // AHEAD: sigma_z of the lines beside this one (groups 2 and 3) was
-            // copied by the CTA's other threads and is in L1, but for the
-            // tile's outer lines
             const int at[6] = {18, rc, 0, 0, rm, rp};
             auto sg = [&](int g, int v) {
-                if (AHEAD && g != 2 && g != 3) return sS[(at[g] + v) * SWX_T];
-                if (!AHEAD && g < 2) return own[6 * g + v];
-                return __ldg(gp[g] + v * TILE3);
+                if (AHEAD) return g == 2 ? hm[v * SWX_T] : g == 3 ? hp[v * SWX_T] : sS[(at[g] + v) * SWX_T];
+                return g < 2 ? own[6 * g + v] : __ldg(gp[g] + v * TILE3);
             };
             sweep_states<R, AMR, 0, OPT>(a, X, sq, dt, c, j, k, Vc, eb, e, vecL, vecR, sg, [] {}, Wm, Wp);
-            if (AHEAD && k + 1 < k1) { // the next plane's, over the ones just used
-                copy_sig(rm, 1, k + 2);
-                copy_sig(18, 2, k + 1);
-                cp_async_commit();
-            }
 #pragma unroll
             for (int q = 0; q < 6; q++) sW[q * SWX_T + t] = Wp[q];
             if (c >= f0 && c < N) {
@@ -526,10 +553,15 @@ __global__ void __launch_bounds__(SWX_T, SwxMinB<R>::value) sweepx3d_kernel(cons
                 w[G.nw(0)] = Wm[P];
             }
         }
+        __syncthreads();
+        if (AHEAD && st && k + 1 < k1) {   // the next plane's sigmas, over the ones just used
+            copy_sig(rm, 1, k + 2);
+            copy_sigz(k + 1);
+            cp_async_commit();
+        }
         {
             const int r = rm; rm = rc; rc = rp; rp = r;
         }
-        __syncthreads();
         if (st && c >= f0) {
             R VL[6], F[NF];
 #pragma unroll
@@ -537,21 +569,20 @@ __global__ void __launch_bounds__(SWX_T, SwxMinB<R>::value) sweepx3d_kernel(cons
             const int er = riemann<R, 0, OPT>(a.prm, 0, VL, (R)V[GC * NWIN + wc - 1], (R)V[GE * NWIN + wc - 1], Wm,
                                          (R)V[GC * NWIN + wc], (R)V[GE * NWIN + wc], F);
             if (er) atomicOr(a.err, er);
-            R *f = X.flx[0] + tile_at<NF>(G.fidx(0, c, j, k));
-#pragma unroll
-            for (int q = 0; q < NF; q++) if (q != FP || fp) f[q * TILE3] = F[q];
+            store_fluxes<R, AMR, 0>(a, X, c, j, k, fp, F);
         }
     }
 }
 
-// The tile: of 1 .. 16 lines per CTA the count with the fewest tiles per
+// The tile: of up to 16 lines per CTA the count with the fewest tiles per
 // plane, the line's faces split evenly over the segments.
 template <class R, int ORDER, bool AMR, int OPT> void launch_sweepx3d(const Args3D &a0, unsigned entries, cudaStream_t s)
 {
     Args3D a = a0;
     constexpr int EX = swx_extra<ORDER>();
     long best = -1;
-    for (int t1 = 1; t1 <= 16; t1 *= 2) {
+    // (two lines at least where the tile's outer lines share rows of SWX_T values)
+    for (int t1 = swx_ahead<R>() ? 2 : 1; t1 <= 16; t1 *= 2) {
         int len = SWX_T / t1 - EX;
         len = len < a.nx + 1 ? len : a.nx + 1;
         if (len < 2 || t1 * (len + 5) > 2 * SWX_T) continue;
@@ -568,7 +599,7 @@ template <class R, int ORDER, bool AMR, int OPT> void launch_sweepx3d(const Args
     a.swx_planes = (int)((a.nz + chunks - 1) / chunks);
     chunks = (a.nz + a.swx_planes - 1) / a.swx_planes;
     const size_t smem = 16 * (size_t)a.swx_lines * (a.swx_len + 5) * (AMR ? sizeof(R) : sizeof(double)) +
-                        ((ORDER == 3 ? 12 : 6) + (swx_ahead<R>() ? 24 : 0)) * (size_t)SWX_T * sizeof(R);
+                        ((ORDER == 3 ? 12 : 6) + (swx_ahead<R>() ? 30 : 0)) * (size_t)SWX_T * sizeof(R);
     if (smem > 48 * 1024)
         cudaFuncSetAttribute(sweepx3d_kernel<R, ORDER, AMR, OPT>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     sweepx3d_kernel<R, ORDER, AMR, OPT><<<dim3((unsigned)best, (unsigned)chunks, entries), SWX_T, smem, s>>>(a);
