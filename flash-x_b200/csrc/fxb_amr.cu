@@ -1383,8 +1383,8 @@ int batched_step(const double *dtv, double dt, int &nl)
     Args3D a = batch_args(dtv, dt);
     auto fluxes = [&](int cnt) {
         const int all = AMR_SIG | AMR_STATES;
-        if (mixed) launch_amr3d_fluxes_mixed(a, cnt, all, S.C.stream);
-        else launch_amr3d_fluxes_fp64(a, cnt, all, S.C.stream);
+        if (mixed) launch_amr3d_fluxes_mixed(a, cnt, all, S.C.stream, S.C.sweeps);
+        else launch_amr3d_fluxes_fp64(a, cnt, all, S.C.stream, S.C.sweeps);
     };
     // the default options' sweeps store the boundary fluxes themselves
     const bool ext = extended_options(S.C.dprm);
@@ -1464,8 +1464,8 @@ int amr_tune()
             fill_batch(a.batch, cnt, S.cur);
             CKA(cudaEventRecord(e[1], S.C.stream));
             for (int st = 0; st < 2; st++) {
-                if (mixed) launch_amr3d_fluxes_mixed(a, cnt, 1 << st, S.C.stream);
-                else launch_amr3d_fluxes_fp64(a, cnt, 1 << st, S.C.stream);
+                if (mixed) launch_amr3d_fluxes_mixed(a, cnt, 1 << st, S.C.stream, S.C.sweeps);
+                else launch_amr3d_fluxes_fp64(a, cnt, 1 << st, S.C.stream, S.C.sweeps);
                 CKA(cudaEventRecord(e[2 + st], S.C.stream));
             }
             if (mixed) launch_amr3d_update_mixed(a, cnt, S.C.stream); else launch_amr3d_update_fp64(a, cnt, S.C.stream);

@@ -7,12 +7,14 @@
 #include <cuda_runtime.h>
 #include "../../include/flashx_b200.h"
 #include "fxb_device.cuh"
+#include "fxb_hydro3d.cuh"
 
 namespace fxb {
 
 // what the AMR mode shares with the rest of the library
 struct AmrCommon {
     cudaStream_t stream;
+    SweepStreams sweeps;          // for the sweeps side by side
     fxb_params prm;
     fxb_domain dom;
     DevParams dprm;

@@ -73,6 +73,7 @@ struct Lib {
     const double *unk_attached = nullptr;
     bool attached = false;
     cudaStream_t stream = nullptr;
+    SweepStreams sweeps{};         // 3-D: for the sweeps side by side
     cudaEvent_t ev0 = nullptr, ev1 = nullptr;
     int last_launches = 0;
     bool timing_valid = false;
@@ -526,8 +527,8 @@ int launch_hydro(int src, const double *dtv, double dt)
         for (int d = 0; d < 3; d++) a.sf_t1[d] = L.sf_t1[d];
         for (int d = 0; d < 3 && L.ns; d++)
             if (cudaMemsetAsync(L.ctufb[d], 0, L.snw, L.stream) != cudaSuccess) return cuda_fail(cudaGetLastError(), "memset");
-        if (L.prm.precision == FXB_MIXED) launch_hydro3d_mixed(a, L.stream);
-        else launch_hydro3d_fp64(a, L.stream);
+        if (L.prm.precision == FXB_MIXED) launch_hydro3d_mixed(a, L.stream, L.sweeps);
+        else launch_hydro3d_fp64(a, L.stream, L.sweeps);
     }
     cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess) return cuda_fail(e, "hydro kernel launch");
@@ -636,6 +637,11 @@ void free_all()
     if (L.mapped_registered) cudaHostUnregister(const_cast<void *>(L.mapped_host));
     if (L.ev0) cudaEventDestroy(L.ev0);
     if (L.ev1) cudaEventDestroy(L.ev1);
+    for (int q = 0; q < 2; q++) {
+        if (L.sweeps.join[q]) cudaEventDestroy(L.sweeps.join[q]);
+        if (L.sweeps.side[q]) cudaStreamDestroy(L.sweeps.side[q]);
+    }
+    if (L.sweeps.fork) cudaEventDestroy(L.sweeps.fork);
     if (L.stream) cudaStreamDestroy(L.stream);
     fxb_error keep = L.lasterr;
     L = Lib();
@@ -811,6 +817,11 @@ extern "C" int fxb_init_slab(const fxb_params *params, const fxb_domain *domain,
         const char *tv = getenv("FXB_TMA");
         L.use_tma = !(tv && tv[0] == '0');
     } else {
+        CK(cudaEventCreateWithFlags(&L.sweeps.fork, cudaEventDisableTiming));
+        for (int q = 0; q < 2; q++) {
+            CK(cudaStreamCreateWithFlags(&L.sweeps.side[q], cudaStreamNonBlocking));
+            CK(cudaEventCreateWithFlags(&L.sweeps.join[q], cudaEventDisableTiming));
+        }
         CK(setup_hydro3d_fp64());
         CK(setup_hydro3d_mixed());
         // intermediates of the unfused 3-D pipeline, in the reconstruction type
@@ -897,7 +908,7 @@ extern "C" int fxb_register_blocks(const fxb_block_desc *blocks, int nblk)
             return fail(FXB_EUNSUPPORTED, "fxb_register_blocks: a slab of a grid takes its level-1 blocks only");
         // block-structured AMR mesh: parents derived, leaves keep their UNK slots
         AmrCommon c;
-        c.stream = L.stream; c.prm = L.prm; c.dom = L.dom; c.dprm = L.dprm; c.nunk = L.nunk;
+        c.stream = L.stream; c.sweeps = L.sweeps; c.prm = L.prm; c.dom = L.dom; c.dprm = L.dprm; c.nunk = L.nunk;
         for (int v = 0; v < NV_DEV; v++) c.dmap[v] = L.dmap[v];
         c.err = L.err; c.rate_max = L.rate_max; c.dtv = L.dtv;
         c.gam1inv = L.gam1inv; c.ggprodinv = L.ggprodinv;

@@ -17,11 +17,12 @@
 //
 // Against slope, face-state and flux kernels (FP64) and the fused tile kernel
 // with two barriers per cell (FP32), 128^3: one direction of PPM FP64 374 ->
-// 257 us along y and z and 398 -> 341 us along x, of WENO5 FP64 470 -> 425 and
+// 257 us along y and z and 398 -> 332 us along x, of WENO5 FP64 470 -> 425 and
 // 456 us, PPM FP32 190 -> 128 and 168 us; without the copies ahead the y and z
-// kernels took 390 us.  Whole steps: PPM 1.40 -> 1.09 ms (mixed 0.73 -> 0.64),
-// WENO5 with gravity 1.61 -> 1.52 (mixed 0.76 -> 0.69), AMR (720 leaves of 16^3)
-// 2.32 -> 1.99 (mixed 1.25 -> 1.08).
+// kernels took 390 us.  Whole steps, with the rest of the step as it is now
+// (sweeps side by side, boundary fluxes from here): PPM 1.40 -> 1.04 ms (mixed
+// 0.73 -> 0.57), WENO5 with gravity 1.61 -> 1.52 (mixed 0.76 -> 0.65), AMR (720
+// leaves of 16^3) 2.32 -> 1.87 (mixed 1.25 -> 0.96).
 #pragma once
 #include "fxb_hydro3d.cuh"
 #include "fxb_tma.cuh"
