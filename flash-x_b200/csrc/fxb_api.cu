@@ -26,6 +26,12 @@ using namespace fxb;
 
 namespace {
 
+struct Status {
+    double dtv[2];
+    unsigned long long rate_max;
+    int err, pad;
+};
+
 struct Lib {
     bool inited = false;
     fxb_params prm{};
@@ -50,6 +56,8 @@ struct Lib {
     int *bcoord = nullptr;         // 3 ints per block
     int *dmap_dev = nullptr;
     int nblk = 0;
+    // the step's scalars, one device record (Status) read back in one copy
+    struct Status *stat = nullptr, *stat_host = nullptr;   // device, page-locked copy
     double *dtv = nullptr;         // [dt, dtOld]
     unsigned long long *rate_max = nullptr;
     int *err = nullptr;
@@ -578,11 +586,17 @@ int ug_step_launches()
     return (L.dom.ndim == 2 ? 1 : hydro3d_launches(L.prm)) + (L.prm.flattening ? 1 : 0) + (L.ns ? 3 : 0);
 }
 
-int check_err_word()
+// the step's scalars into the page-locked record, after the stream's work
+int read_status()
 {
-    int h = 0;
-    CK(cudaMemcpyAsync(&h, L.err, sizeof(int), cudaMemcpyDeviceToHost, L.stream));
+    CK(cudaMemcpyAsync(L.stat_host, L.stat, sizeof(Status), cudaMemcpyDeviceToHost, L.stream));
     CK(cudaStreamSynchronize(L.stream));
+    return FXB_OK;
+}
+// the record's error word as a status code; a set word is cleared on the device
+int status_error()
+{
+    const int h = L.stat_host->err;
     if (h) {
         CK(cudaMemsetAsync(L.err, 0, sizeof(int), L.stream));
         if (h & ERR_SOUND)
@@ -594,6 +608,11 @@ int check_err_word()
         return fail(FXB_ECUDA, "device error word set");
     }
     return FXB_OK;
+}
+int check_err_word()
+{
+    const int rc = read_status();
+    return rc ? rc : status_error();
 }
 
 void free_all()
@@ -621,10 +640,9 @@ void free_all()
     if (L.pmap_dev) cudaFree(L.pmap_dev);
     if (L.pack_dev) cudaFree(L.pack_dev);
     if (L.pack_host) cudaFreeHost(L.pack_host);
-    if (L.dtv) cudaFree(L.dtv);
+    if (L.stat) cudaFree(L.stat);
+    if (L.stat_host) cudaFreeHost(L.stat_host);
     if (L.shok) cudaFree(L.shok);
-    if (L.rate_max) cudaFree(L.rate_max);
-    if (L.err) cudaFree(L.err);
     if (L.partials) cudaFree(L.partials);
     if (L.sig3) cudaFree(L.sig3);
     if (L.slp3) cudaFree(L.slp3);
@@ -782,15 +800,16 @@ extern "C" int fxb_init_slab(const fxb_params *params, const fxb_domain *domain,
     CK(cudaMalloc(&L.dmap_dev, sizeof(int) * NV_DEV));
     CK(cudaMalloc(&L.pmap_dev, sizeof(int) * NV_DEV));
     CK(cudaMemcpyAsync(L.dmap_dev, L.dmap, sizeof(int) * NV_DEV, cudaMemcpyHostToDevice, L.stream));
-    CK(cudaMalloc(&L.dtv, 2 * sizeof(double)));
+    CK(cudaMalloc(&L.stat, sizeof(Status)));
+    CK(cudaMallocHost(&L.stat_host, sizeof(Status)));
+    CK(cudaMemsetAsync(L.stat, 0, sizeof(Status), L.stream));
+    L.dtv = L.stat->dtv;
+    L.rate_max = &L.stat->rate_max;
+    L.err = &L.stat->err;
     if (L.dprm.shock_detect) {
         CK(cudaMalloc(&L.shok, (size_t)L.vstride));
         CK(cudaMemsetAsync(L.shok, 0, (size_t)L.vstride, L.stream));
     }
-    CK(cudaMalloc(&L.rate_max, sizeof(unsigned long long)));
-    CK(cudaMalloc(&L.err, sizeof(int)));
-    CK(cudaMemsetAsync(L.err, 0, sizeof(int), L.stream));
-    CK(cudaMemsetAsync(L.rate_max, 0, sizeof(unsigned long long), L.stream));
     L.npartials = 1024;
     CK(cudaMalloc(&L.partials, sizeof(double) * (L.npartials * 7 + 8)));
     if (q.use_gravity) {   // gravity's face values, once, in each precision's kernels' arithmetic
@@ -1110,7 +1129,6 @@ extern "C" int fxb_sync_to_host(double *unk_host)
         shok_to_unk_kernel<<<1184, 256, 0, L.stream>>>(L.shok, L.unk_dev, g, L.bcoord, L.nblk, L.shock_slot);
     CK(cudaGetLastError());
     CK(cudaMemcpyAsync(unk_host, L.unk_dev, sizeof(double) * L.unk_doubles, cudaMemcpyDeviceToHost, L.stream));
-    CK(cudaStreamSynchronize(L.stream));
     L.counts[FXB_COUNT_GC_FILLS]++;
     L.counts[FXB_COUNT_GC_DOUBLES] += L.unk_doubles;
     return check_err_word();
@@ -1235,7 +1253,6 @@ extern "C" int fxb_put_interior(const double *unk_host)
     if (L.ns)
         unk_to_spec_kernel<<<1184, 256, 0, L.stream>>>(L.unk_dev, L.spb[L.cur], g, L.bcoord, L.sslot_dev, L.ns, L.nblk);
     CK(cudaGetLastError());
-    CK(cudaStreamSynchronize(L.stream));
     state_changed(false);
     L.shok_valid = false;         // the host's SHOK stands until the next step
     return check_err_word();
@@ -1256,9 +1273,7 @@ extern "C" int fxb_get_interior(double *unk_host)
         shok_to_unk_kernel<<<1184, 256, 0, L.stream>>>(L.shok, L.unk_dev, g, L.bcoord, L.nblk, L.shock_slot);
     CK(cudaGetLastError());
     rc = copy_interior_rows(unk_host, L.unk_dev, cudaMemcpyDeviceToHost);
-    if (rc) return rc;
-    CK(cudaStreamSynchronize(L.stream));
-    return check_err_word();
+    return rc ? rc : check_err_word();
 }
 
 namespace {
@@ -1421,7 +1436,7 @@ extern "C" int fxb_compute_dt(double *dt_out, int32_t loc[5])
         CK(cudaGetLastError());
         L.rate_valid = true;
     }
-    unsigned long long bits = 0, key = ~0ull;
+    unsigned long long key = ~0ull;
     if (loc) {
         // L.partials doubles as the 8-byte key (fxb_integrals rewrites it before use)
         unsigned long long *dkey = (unsigned long long *)L.partials;
@@ -1438,10 +1453,9 @@ extern "C" int fxb_compute_dt(double *dt_out, int32_t loc[5])
         }
         CK(cudaMemcpyAsync(&key, dkey, sizeof(key), cudaMemcpyDeviceToHost, L.stream));
     }
-    CK(cudaMemcpyAsync(&bits, L.rate_max, sizeof(bits), cudaMemcpyDeviceToHost, L.stream));
-    CK(cudaStreamSynchronize(L.stream));
     int rc = check_err_word();
     if (rc) return rc;
+    const unsigned long long bits = L.stat_host->rate_max;
     double r;
     memcpy(&r, &bits, sizeof(r));
     double dt = (r != 0.) ? L.prm.cfl / r : 1.79769313486231570e308;
@@ -1475,9 +1489,8 @@ extern "C" int fxb_advance(int nsteps, double *dt, double *dt_old, double f, dou
     if (!L.attached) return fail(FXB_EARG, "fxb_advance: no UNK attached");
     if (!dt || !dt_old || nsteps < 0) return fail(FXB_EARG, "fxb_advance: bad argument");
     if (has_halo()) return fail(FXB_EUNSUPPORTED, "fxb_advance: a slab with halos exchanges them between steps");
-    double h[2] = {*dt, *dt_old};
-    CK(cudaMemcpyAsync(L.dtv, h, sizeof(h), cudaMemcpyHostToDevice, L.stream));
-    CK(cudaMemsetAsync(L.rate_max, 0, sizeof(unsigned long long), L.stream));
+    const double h[3] = {*dt, *dt_old, 0.};       // dt, dtOld and the CFL rate's start
+    CK(cudaMemcpyAsync(L.stat, h, sizeof(h), cudaMemcpyHostToDevice, L.stream));
     // graphs of two steps (buffer c -> 1-c -> c), built once per starting buffer
     const bool amr = amr_active();
     int step_launches = amr ? 0 : ug_step_launches();
@@ -1512,15 +1525,15 @@ extern "C" int fxb_advance(int nsteps, double *dt, double *dt_old, double f, dou
         if (!amr) L.cur = 1 - L.cur;
     }
     CK(cudaEventRecord(L.ev1, L.stream));
-    CK(cudaMemcpyAsync(h, L.dtv, sizeof(h), cudaMemcpyDeviceToHost, L.stream));
-    CK(cudaStreamSynchronize(L.stream));
-    *dt = h[0];
-    *dt_old = h[1];
+    const int rrc = read_status();
+    if (rrc) return rrc;
+    *dt = L.stat_host->dtv[0];
+    *dt_old = L.stat_host->dtv[1];
     state_changed(false);
     L.counts[FXB_COUNT_STEPS] += nsteps;
     L.last_launches = (step_launches + 1) * nsteps;
     L.timing_valid = true;
-    return check_err_word();
+    return status_error();
 }
 
 extern "C" int fxb_integrals(double out[7])
