@@ -1196,10 +1196,13 @@ __global__ void __launch_bounds__(256) interior_rows_kernel(T *__restrict__ dst,
 // the interior rows of every block, between the caller's UNK and the device
 // mirror.  2-D: one strided copy over all blocks (their rows are evenly
 // spaced).  3-D: the k guard planes separate the blocks, so the copy engine
-// would need a copy per block, 6 us of host time each (2,805 blocks of 8^3,
-// 126 MB: 17 ms each way against 2.5 ms of bus time); one kernel reads or
-// writes the page-locked memory instead.  Memory that the device cannot
-// address keeps the copies.
+// needs a copy per block, 6 us of host time each (2,805 blocks of 8^3, 126 MB:
+// 17 ms each way against 2.5 ms of bus time); blocks below kRowsKernelBytes go
+// by one kernel that reads or writes the page-locked memory.  The line lies
+// between the sizes measured, put + get: 8^3 blocks (45 KB) 35 -> 10 ms, 16^3
+// (360 KB, 128^3 cells) 11.1 -> 9.3 ms, 32^3 (2.9 MB, 192^3 cells) 25.7 -> 27.7 ms.
+// Memory that the device cannot address keeps the copies.
+constexpr size_t kRowsKernelBytes = 1u << 20;
 int copy_interior_rows(double *dst, const double *src, cudaMemcpyKind kind)
 {
     const UnkGeom g = unk_geom();
@@ -1217,7 +1220,7 @@ int copy_interior_rows(double *dst, const double *src, cudaMemcpyKind kind)
     }
     const bool in = kind == cudaMemcpyHostToDevice;
     void *host = nullptr;
-    if (cudaHostGetDevicePointer(&host, in ? const_cast<double *>(src) : dst, 0) == cudaSuccess && host) {
+    if (w * g.nyb * g.nzb < kRowsKernelBytes && cudaHostGetDevicePointer(&host, in ? const_cast<double *>(src) : dst, 0) == cudaSuccess && host) {
         double *kd = in ? dst : (double *)host;
         const double *ks = in ? (const double *)host : src;
         // 16-byte elements where rows, pitches and the guard cells before a row are whole pairs of values

@@ -127,8 +127,10 @@ def test_amr_option_matches_oracle(oracle, need_gpu, name):
     _check(out, ref[:, g:-g, g:-g, g:-g][..., HYDRO_VARS])
 
 
-# rows of whole 16-byte pairs, and (odd block sizes, odd slot counts) not
-@pytest.mark.parametrize("n", [8, 5])
+# rows of whole 16-byte pairs, and (odd block sizes, odd slot counts) not;
+# blocks of 935,088 and 1,068,672 bytes on both sides of the 1 MiB from which
+# the copy engine moves them
+@pytest.mark.parametrize("n", [8, 5, 21, 22])
 def test_3d_interior_transfers_move_every_row(need_gpu, n):
     geom = Geometry(3, n, n + 1, n + 2, 3, 2, 2, bc=(BC_PERIODIC,) * 6)
     hp = HydroParams()
