@@ -1201,8 +1201,34 @@ __global__ void __launch_bounds__(256) interior_rows_kernel(T *__restrict__ dst,
 // by one kernel that reads or writes the page-locked memory.  The line lies
 // between the sizes measured, put + get: 8^3 blocks (45 KB) 35 -> 10 ms, 16^3
 // (360 KB, 128^3 cells) 11.1 -> 9.3 ms, 32^3 (2.9 MB, 192^3 cells) 25.7 -> 27.7 ms.
-// Memory that the device cannot address keeps the copies.
+// Memory that the device cannot address as doubles keeps the copies.
 constexpr size_t kRowsKernelBytes = 1u << 20;
+
+// Whether kernels can read and write all of [p, p + bytes) as doubles: the
+// address is a multiple of 8, and the page-locked range it lies in (the
+// caller's own may be another one than the array) reaches to the array's end.
+// *dev: the array's device address.
+bool device_addressable(void *p, size_t bytes, void **dev)
+{
+    static PFN_cuPointerGetAttribute_v4000 get = nullptr;
+    if ((uintptr_t)p % sizeof(double)) return false;
+    if (!get) {
+        void *fn = nullptr;
+        cudaDriverEntryPointQueryResult q = cudaDriverEntryPointSymbolNotFound;
+        if (cudaGetDriverEntryPoint("cuPointerGetAttribute", &fn, cudaEnableDefault, &q) == cudaSuccess &&
+            q == cudaDriverEntryPointSuccess)
+            get = (PFN_cuPointerGetAttribute_v4000)fn;
+    }
+    CUdeviceptr start = 0;
+    size_t size = 0;
+    const bool whole = get && get(&start, CU_POINTER_ATTRIBUTE_RANGE_START_ADDR, (CUdeviceptr)p) == CUDA_SUCCESS &&
+                       get(&size, CU_POINTER_ATTRIBUTE_RANGE_SIZE, (CUdeviceptr)p) == CUDA_SUCCESS &&
+                       (CUdeviceptr)p >= start && (CUdeviceptr)p - start <= size &&
+                       bytes <= size - ((CUdeviceptr)p - start);
+    const bool ok = whole && cudaHostGetDevicePointer(dev, p, 0) == cudaSuccess && *dev;
+    cudaGetLastError();
+    return ok;
+}
 int copy_interior_rows(double *dst, const double *src, cudaMemcpyKind kind)
 {
     const UnkGeom g = unk_geom();
@@ -1220,7 +1246,8 @@ int copy_interior_rows(double *dst, const double *src, cudaMemcpyKind kind)
     }
     const bool in = kind == cudaMemcpyHostToDevice;
     void *host = nullptr;
-    if (w * g.nyb * g.nzb < kRowsKernelBytes && cudaHostGetDevicePointer(&host, in ? const_cast<double *>(src) : dst, 0) == cudaSuccess && host) {
+    if (w * g.nyb * g.nzb < kRowsKernelBytes &&
+        device_addressable(in ? const_cast<double *>(src) : dst, sizeof(double) * L.unk_doubles, &host)) {
         double *kd = in ? dst : (double *)host;
         const double *ks = in ? (const double *)host : src;
         // 16-byte elements where rows, pitches and the guard cells before a row are whole pairs of values
@@ -1233,7 +1260,6 @@ int copy_interior_rows(double *dst, const double *src, cudaMemcpyKind kind)
         CK(cudaGetLastError());
         return FXB_OK;
     }
-    cudaGetLastError();
     p.extent = make_cudaExtent(w, g.nyb, g.nzb);
     for (int b = 0; b < L.nblk; b++) {
         p.srcPos = p.dstPos = make_cudaPos(x0, g.ng, (size_t)b * g.nkg + g.ng);

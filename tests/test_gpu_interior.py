@@ -190,3 +190,59 @@ def test_a_replaced_device_refuses_calls(need_gpu):
     b.close()
     with pytest.raises(FlashXError):
         b.Hydro_computeDt()
+
+
+# Blocks small enough for the kernel over page-locked memory, in arrays that it
+# must not read as they are: it takes doubles at multiples of 8 bytes inside
+# one page-locked range, and everything else goes by the copy engine.
+def _small_blocks():
+    geom = Geometry(3, 8, 8, 8, 3, 2, 2, bc=(BC_PERIODIC,) * 6)
+    hp = HydroParams()
+    return geom, hp, S.noisy_gas(geom, hp)
+
+
+@pytest.mark.parametrize("shift", [0, 1, 4, 8])
+def test_interior_transfers_of_arrays_at_any_address(need_gpu, shift):
+    geom, hp, unk = _small_blocks()
+    raw = [np.zeros(unk.nbytes + 64, dtype=np.uint8) for _ in range(2)]
+    src, dst = (r[-r.ctypes.data % 16 + shift:][:unk.nbytes].view(np.float64).reshape(unk.shape) for r in raw)
+    assert src.ctypes.data % 16 == shift and dst.ctypes.data % 16 == shift
+    src[...] = unk
+    src[..., DENS] *= 2.0
+    dst[...] = -7.0
+    dev = HydroDevice(geom, hp, "fp64")
+    dev.attach_unk(unk.copy())
+    dev.put_interior(src)
+    dev.get_interior(dst)
+    dev.close()
+    assert np.array_equal(_interior(geom, dst)[..., DEV_VARS], _interior(geom, src)[..., DEV_VARS])
+
+
+@pytest.mark.parametrize("share", [0.5, 1.0])
+def test_interior_transfers_of_an_array_the_caller_page_locked(need_gpu, share):
+    """All of it, or (one mistake away) its first half only: the transfer
+    then moves every row or raises, and the device stays usable."""
+    import torch
+    geom, hp, unk = _small_blocks()
+    rt = torch.cuda.cudart()
+    torch.cuda.init()
+    src = unk.copy()
+    src[..., DENS] *= 2.0
+    n = int(src.nbytes * share) // 4096 * 4096 if share < 1.0 else src.nbytes
+    dev = HydroDevice(geom, hp, "fp64")
+    dev.attach_unk(unk.copy())
+    assert int(rt.cudaHostRegister(src.ctypes.data, n, 0)) == 0
+    try:
+        moved = True
+        try:
+            dev.put_interior(src)
+        except FlashXError:
+            moved = False
+            dev.put_interior(unk.copy())
+        dst = np.zeros(unk.shape)
+        dev.get_interior(dst)
+    finally:
+        dev.close()
+        assert int(rt.cudaHostUnregister(src.ctypes.data)) == 0
+    assert moved or share < 1.0
+    assert np.array_equal(_interior(geom, dst)[..., DEV_VARS], _interior(geom, src if moved else unk)[..., DEV_VARS])
