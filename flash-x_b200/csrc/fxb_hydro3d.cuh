@@ -836,8 +836,14 @@ __device__ __forceinline__ void flux3d_kernel_body(const Args3D &a, const VB vb)
         for (int q = 0; q < NF; q++) o[q * TILE3] = F[q];
     }
 }
+// Two CTAs per SM: with the 137 to 153 registers that some instantiations took
+// one was left, and a direction of the extended options' fluxes 63 to 110 us at
+// 80^3 (artificial viscosity; Roe 26 to 40).  A step at 80^3, with 128 registers
+// and up to 84 bytes of spills: artificial viscosity 521 -> 476 us, Roe 387 ->
+// 375, MarquinaModified 419 -> 391, AMR with viscosity (288 leaves of 16^3) 1,276 ->
+// 1,121.
 template <class R, bool AMR, int DIR, int EXT>
-__global__ void __launch_bounds__(256) flux3d_kernel(const Args3D a)
+__global__ void __launch_bounds__(256, 2) flux3d_kernel(const Args3D a)
 {
     flux3d_kernel_body<R, AMR, DIR, EXT>(a, hw_block());
 }
