@@ -721,6 +721,13 @@ __device__ __noinline__ WenoPair<R> weno_scalar_body(int method, R I0, R I1, R I
     const R s[2] = {a[0] + a[1] + a[2], c[0] + c[1] + c[2]};
     R ys[2];
     recips(s, ys);
+    if constexpr (sizeof(R) == 4) {
+        // the middle weight as one minus the other two: the rounding of the
+        // weights then multiplies differences of the candidates and not the
+        // candidates themselves
+        return WenoPair<R>{w5p1 + rdiv_y(a[0], s[0], ys[0]) * (w5p0 - w5p1) + rdiv_y(a[2], s[0], ys[0]) * (w5p2 - w5p1),
+                           w5m1 + rdiv_y(c[0], s[1], ys[1]) * (w5m0 - w5m1) + rdiv_y(c[2], s[1], ys[1]) * (w5m2 - w5m1)};
+    }
     const R vr = rdiv_y(a[0], s[0], ys[0]) * w5p0 + rdiv_y(a[1], s[0], ys[0]) * w5p1 + rdiv_y(a[2], s[0], ys[0]) * w5p2;
     const R vl = rdiv_y(c[0], s[1], ys[1]) * w5m0 + rdiv_y(c[1], s[1], ys[1]) * w5m1 + rdiv_y(c[2], s[1], ys[1]) * w5m2;
     return WenoPair<R>{vr, vl};
