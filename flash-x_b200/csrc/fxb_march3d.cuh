@@ -144,28 +144,28 @@ __device__ __forceinline__ void store_fluxes(const Args3D &a, const Ctx3<R, AMR>
     }
 }
 
-constexpr int MARCH_T = 128;          // threads per CTA
-// resident CTAs per SM: 168 registers per thread in FP64 (shared memory allows
-// no fourth CTA), 96 in FP32 (six CTAs of 80 registers: PPM 128^3 0.66 instead
-// of 0.64 ms)
+// CTAs of T threads: 128, or on AMR leaves 64 where fewer threads are then
+// without a line (8^3 leaves have 64 lines, 12^3 ones 144).  Resident CTAs per
+// SM for 128 threads each: 168 registers per thread in FP64 (shared memory
+// allows no fourth CTA), 96 in FP32 (six CTAs of 80 registers: PPM 128^3 0.66
+// instead of 0.64 ms)
 #ifndef FXB_MARCH_MINB64
 #define FXB_MARCH_MINB64 3
 #endif
 #ifndef FXB_MARCH_MINB32
 #define FXB_MARCH_MINB32 5
 #endif
-template <class R> struct MarchMinB { static constexpr int value = sizeof(R) == 8 ? FXB_MARCH_MINB64 : FXB_MARCH_MINB32; };
+template <class R, int T> constexpr int march_resident()
+{ return (sizeof(R) == 8 ? FXB_MARCH_MINB64 : FXB_MARCH_MINB32) * 128 / T; }
 // per-thread slots: the stencil's cells (PPM 3, WENO5 5, six values each), two
 // slopes (PPM), the previous cell's right-face state
 template <int ORDER> struct MarchSlots {
     static constexpr int cells = ORDER == 5 ? 5 : 3;
     static constexpr int slope = cells * 6, wp = slope + (ORDER == 5 ? 0 : 12), sig = wp + 6, value = sig + 36;
 };
-template <class R, int ORDER> constexpr int march_smem_bytes()
-{ return MarchSlots<ORDER>::value * MARCH_T * (int)sizeof(R); }
 
-template <class R, int ORDER, bool AMR, int DIR, int OPT>
-__global__ void __launch_bounds__(MARCH_T, MarchMinB<R>::value) march3d_kernel(const Args3D a)
+template <class R, int ORDER, bool AMR, int DIR, int OPT, int T>
+__global__ void __launch_bounds__(T, march_resident<R, T>()) march3d_kernel(const Args3D a)
 {
     static_assert(DIR == 1 || DIR == 2, "lines along y or z");
     extern __shared__ __align__(16) unsigned char march_smem[];
@@ -186,7 +186,7 @@ __global__ void __launch_bounds__(MARCH_T, MarchMinB<R>::value) march3d_kernel(c
     __syncthreads();
     const bool fp = a.prm.fpres != 1.0;            // else the update does not read the pressure slot
     const int N = DIR == 1 ? a.ny : a.nz, N2 = DIR == 1 ? a.nz : a.ny;
-    const int line = (int)(blockIdx.x * MARCH_T + threadIdx.x);
+    const int line = (int)(blockIdx.x * T + threadIdx.x);
     if (line >= a.nx * N2) return;
     const int t2 = (int)fast_div((unsigned)line, a.fdx[0]), i = line - t2 * a.nx;
     const int f0 = (int)blockIdx.y * a.march_len, f1 = min(f0 + a.march_len, N + 1);
@@ -230,11 +230,11 @@ __global__ void __launch_bounds__(MARCH_T, MarchMinB<R>::value) march3d_kernel(c
     using SL = MarchSlots<ORDER>;
     auto put = [&](int slot, const R v[6]) {
 #pragma unroll
-        for (int q = 0; q < 6; q++) sl[(slot + q) * MARCH_T] = v[q];
+        for (int q = 0; q < 6; q++) sl[(slot + q) * T] = v[q];
     };
     auto get = [&](int slot, R v[6]) {
 #pragma unroll
-        for (int q = 0; q < 6; q++) v[q] = sl[(slot + q) * MARCH_T];
+        for (int q = 0; q < 6; q++) v[q] = sl[(slot + q) * T];
     };
 
     // ring of the stencil's cells: ring[0] is the oldest
@@ -279,7 +279,7 @@ __global__ void __launch_bounds__(MARCH_T, MarchMinB<R>::value) march3d_kernel(c
                 if (g >= 2 && !a.prm.use_3d_full_ctu) continue;
                 const R *p = sweep_sig_at<DIR>((const R *)X.sig, G, g, i, j, k);
 #pragma unroll
-                for (int v = 0; v < 6; v++) cp_async(sl + (SL::sig + 6 * g + v) * MARCH_T, p + v * TILE3);
+                for (int v = 0; v < 6; v++) cp_async(sl + (SL::sig + 6 * g + v) * T, p + v * TILE3);
             }
             cp_async_commit();
         }
@@ -320,12 +320,12 @@ __global__ void __launch_bounds__(MARCH_T, MarchMinB<R>::value) march3d_kernel(c
             get(ring[2], Vc);
             if (!eigen_base(Vc[0], Vc[4], gc, ebc)) atomicOr(a.err, ERR_SOUND);
             eigen_dir(ebc, Vc[1], e);
-            weno_interfaces_of<R, OPT>(a.prm, e, [&](int v, int o) { return sl[(ring[o] + v) * MARCH_T]; }, vecL, vecR);
+            weno_interfaces_of<R, OPT>(a.prm, e, [&](int v, int o) { return sl[(ring[o] + v) * T]; }, vecL, vecR);
             const int r0 = ring[0];
             ring[0] = ring[1]; ring[1] = ring[2]; ring[2] = ring[3]; ring[3] = ring[4]; ring[4] = r0;
         }
         sweep_states<R, AMR, DIR, OPT>(a, X, sq, dt, i, j, k, Vc, ebc, e, vecL, vecR,
-                                       [&](int g, int v) { return sl[(SL::sig + 6 * g + v) * MARCH_T]; },
+                                       [&](int g, int v) { return sl[(SL::sig + 6 * g + v) * T]; },
                                        [] { cp_async_wait(); }, Wm, Wp);
         if (c >= f0 && c < N) {
             R *w = X.wst[DIR] + G.widx(DIR, i, j, k);
@@ -356,19 +356,22 @@ inline int cut_line(int len, int least, double extra, long units, long resident)
 #ifndef FXB_MARCH_SMIN
 #define FXB_MARCH_SMIN 3
 #endif
-template <class R, int ORDER, bool AMR, int DIR, int OPT>
-void launch_march3d(const Args3D &a0, unsigned entries, cudaStream_t s)
+// how one sweep is launched
+struct SweepPlan {
+    dim3 grid;
+    int threads;
+    size_t smem;
+    double waves;              // its CTAs over those the chip holds at a time
+};
+template <class R, int ORDER, int DIR, int T> SweepPlan plan_march3d(Args3D &a, unsigned entries)
 {
-    Args3D a = a0;
     const int N = DIR == 1 ? a.ny : a.nz, N2 = DIR == 1 ? a.nz : a.ny;
-    const long ctas = ((long)a.nx * N2 + MARCH_T - 1) / MARCH_T;
-    long nseg = cut_line(N + 1, FXB_MARCH_SMIN, 1.5, ctas * entries, 148L * MarchMinB<R>::value);
+    const long ctas = ((long)a.nx * N2 + T - 1) / T, resident = 148L * march_resident<R, T>();
+    long nseg = cut_line(N + 1, FXB_MARCH_SMIN, 1.5, ctas * entries, resident);
     a.march_len = (int)((N + nseg) / nseg);
     nseg = (N + a.march_len) / a.march_len;
-    constexpr int smem = march_smem_bytes<R, ORDER>();
-    if (smem > 48 * 1024)
-        cudaFuncSetAttribute(march3d_kernel<R, ORDER, AMR, DIR, OPT>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
-    march3d_kernel<R, ORDER, AMR, DIR, OPT><<<dim3((unsigned)ctas, (unsigned)nseg, entries), MARCH_T, smem, s>>>(a);
+    return {dim3((unsigned)ctas, (unsigned)nseg, entries), T, MarchSlots<ORDER>::value * T * sizeof(R),
+            (double)ctas * nseg * entries / resident};
 }
 
 // ---- x sweep -------------------------------------------------------------------
@@ -379,7 +382,6 @@ void launch_march3d(const Args3D &a0, unsigned entries, cudaStream_t s)
 // last), the limited slopes and the right-face states pass through shared
 // memory, with a barrier after each.  The window of the next plane is copied
 // into the second buffer (cp.async) while this one is worked on.
-constexpr int SWX_T = 160;
 #ifndef FXB_SWX_PMIN
 #define FXB_SWX_PMIN 2
 #endif
@@ -389,7 +391,9 @@ constexpr int SWX_T = 160;
 #ifndef FXB_SWX_MINB32
 #define FXB_SWX_MINB32 5
 #endif
-template <class R> struct SwxMinB { static constexpr int value = sizeof(R) == 8 ? FXB_SWX_MINB64 : FXB_SWX_MINB32; };
+// CTAs of T threads: 160, or on AMR leaves 96 where a leaf's tiles then take
+// fewer threads (8^3: one tile of 96); resident CTAs per SM
+template <class R, int T> constexpr int swx_resident() { return (sizeof(R) == 8 ? FXB_SWX_MINB64 : FXB_SWX_MINB32) * 160 / T; }
 // cells per line and tile beyond its faces: one more face state, and with PPM two more slopes
 template <int ORDER> constexpr int swx_extra() { return ORDER == 3 ? 3 : 1; }
 // FP64 copies the sigmas of the next plane into shared memory while it works
@@ -398,8 +402,8 @@ template <int ORDER> constexpr int swx_extra() { return ORDER == 3 ? 3 : 1; }
 // them (RT 128^3 0.69 ms, 0.71 with the copies)
 template <class R> constexpr bool swx_ahead() { return sizeof(R) == 8; }
 
-template <class R, int ORDER, bool AMR, int OPT>
-__global__ void __launch_bounds__(SWX_T, SwxMinB<R>::value) sweepx3d_kernel(const Args3D a)
+template <class R, int ORDER, bool AMR, int OPT, int T>
+__global__ void __launch_bounds__(T, swx_resident<R, T>()) sweepx3d_kernel(const Args3D a)
 {
     using S = typename std::conditional<AMR, R, double>::type;    // type of the source arrays
     constexpr int EX = swx_extra<ORDER>();
@@ -412,14 +416,14 @@ __global__ void __launch_bounds__(SWX_T, SwxMinB<R>::value) sweepx3d_kernel(cons
     const double dt = a.dtv ? a.dtv[0] : a.dt_arg;
     const int T1 = a.swx_lines, Lx = a.swx_len, W = Lx + 5, NWIN = T1 * W, Lt = Lx + EX;
     S *const sV = reinterpret_cast<S *>(swx_smem);                // [2][8][T1][W]
-    R *const sD = reinterpret_cast<R *>(sV + 16 * NWIN);          // PPM: [6][SWX_T] slopes
-    R *const sW = sD + (ORDER == 3 ? 6 * SWX_T : 0);              // [6][SWX_T] right-face states
+    R *const sD = reinterpret_cast<R *>(sV + 16 * NWIN);          // PPM: [6][T] slopes
+    R *const sW = sD + (ORDER == 3 ? 6 * T : 0);              // [6][T] right-face states
     // this thread's sigmas: sigma_y of the planes k - 1, k, k + 1 (six values
     // each, in turn), then sigma_z of plane k
-    R *const sS = sW + 6 * SWX_T + threadIdx.x;
+    R *const sS = sW + 6 * T + threadIdx.x;
     // sigma_z of plane k of the lines before the tile's first and behind its
-    // last one, [6][two lines of Lt cells in rows of SWX_T]
-    R *const sH = sW + 30 * SWX_T;
+    // last one, [6][two lines of Lt cells in rows of T]
+    R *const sH = sW + 30 * T;
     if (t < 5)
         sq[t] = t == 0 ? dt / X.dx
                 : t == 1 ? 0.5 * dt / X.dx
@@ -430,14 +434,14 @@ __global__ void __launch_bounds__(SWX_T, SwxMinB<R>::value) sweepx3d_kernel(cons
     const int N = a.nx, N1 = a.ny, nseg = a.swx_segs;
     const int seg = blockIdx.x % nseg, f0 = seg * Lx, j0 = (blockIdx.x / nseg) * T1;
     const int k0 = blockIdx.y * a.swx_planes, k1 = min(k0 + a.swx_planes, a.nz);
-    // copies of one plane's window: thread t takes window cells t and t + SWX_T
+    // copies of one plane's window: thread t takes window cells t and t + T
     // (cells behind the line's last one or beyond the last line repeat them)
     const S *src;
     if constexpr (AMR) src = X.srcR; else src = X.src;
     long woff[2];
 #pragma unroll
     for (int q = 0; q < 2; q++) {
-        const int w = min(t + q * SWX_T, NWIN - 1), l = w / W;
+        const int w = min(t + q * T, NWIN - 1), l = w / W;
         int x = min(f0 - 3 + w - l * W, N + 2);
         const int y = min(j0 + l, N1 - 1);
         double s_ = 1.0;
@@ -448,7 +452,7 @@ __global__ void __launch_bounds__(SWX_T, SwxMinB<R>::value) sweepx3d_kernel(cons
         const long z = (long)(k + X.so) * X.sy * X.sx;
 #pragma unroll
         for (int q = 0; q < 2; q++) {
-            const int w = t + q * SWX_T;
+            const int w = t + q * T;
             if (w < NWIN) {
 #pragma unroll
                 for (int v = 0; v < 8; v++) cp_async(sV + (buf * 8 + v) * NWIN + w, src + (v * X.svs + z + woff[q]));
@@ -474,12 +478,12 @@ __global__ void __launch_bounds__(SWX_T, SwxMinB<R>::value) sweepx3d_kernel(cons
     auto copy_sig = [&](int slot, int d, int k) {
         const R *p = (const R *)X.sig + tile_at<NSIG>(G.pidx(c, j, k)) + 6 * d * TILE3;
 #pragma unroll
-        for (int v = 0; v < 6; v++) cp_async(sS + (slot + v) * SWX_T, p + v * TILE3);
+        for (int v = 0; v < 6; v++) cp_async(sS + (slot + v) * T, p + v * TILE3);
     };
     int rm = 0, rc = 6, rp = 12;       // slots of sigma_y of the planes k - 1, k, k + 1
     // sigma_z beside this line: the neighbour thread's own, or the outer lines'
     const bool first = l1 == 0, last = l1 + 1 == T1 || j + 1 == N1;
-    const R *const hm = first ? sH + ld : sS - Lt + 18 * SWX_T, *const hp = last ? sH + Lt + ld : sS + Lt + 18 * SWX_T;
+    const R *const hm = first ? sH + ld : sS - Lt + 18 * T, *const hp = last ? sH + Lt + ld : sS + Lt + 18 * T;
     auto copy_sigz = [&](int k) {
         copy_sig(18, 2, k);
 #pragma unroll
@@ -487,7 +491,7 @@ __global__ void __launch_bounds__(SWX_T, SwxMinB<R>::value) sweepx3d_kernel(cons
             if (side ? !last : !first) continue;
             const R *p = sweep_sig_at<0>((const R *)X.sig, G, 2 + side, c, j, k);
 #pragma unroll
-            for (int v = 0; v < 6; v++) cp_async(sH + v * SWX_T + side * Lt + ld, p + v * TILE3);
+            for (int v = 0; v < 6; v++) cp_async(sH + v * T + side * Lt + ld, p + v * TILE3);
         }
     };
     copy_plane(k0, 0);
@@ -513,7 +517,7 @@ __global__ void __launch_bounds__(SWX_T, SwxMinB<R>::value) sweepx3d_kernel(cons
                 eigen_dir(eb, Vc[1], e);
                 tvd_slope<R, OPT>(a.prm, e, Vm, Vc, Vp, db);
 #pragma unroll
-                for (int q = 0; q < 6; q++) sD[q * SWX_T + t] = db[q];
+                for (int q = 0; q < 6; q++) sD[q * T + t] = db[q];
             }
             __syncthreads();
             if (st) {
@@ -521,7 +525,7 @@ __global__ void __launch_bounds__(SWX_T, SwxMinB<R>::value) sweepx3d_kernel(cons
                 six_at(V, -1, Vm); six_at(V, 1, Vp);
 #pragma unroll
                 for (int q = 0; q < 6; q++) {
-                    dbN[q] = sD[q * SWX_T + t - 1]; db0[q] = sD[q * SWX_T + t]; dbP[q] = sD[q * SWX_T + t + 1];
+                    dbN[q] = sD[q * T + t - 1]; db0[q] = sD[q * T + t]; dbP[q] = sD[q * T + t + 1];
                 }
                 ppm_interfaces(Vm, Vc, Vp, dbN, db0, dbP, vecL, vecR);
             }
@@ -542,12 +546,12 @@ __global__ void __launch_bounds__(SWX_T, SwxMinB<R>::value) sweepx3d_kernel(cons
             }
             const int at[6] = {18, rc, 0, 0, rm, rp};
             auto sg = [&](int g, int v) {
-                if (AHEAD) return g == 2 ? hm[v * SWX_T] : g == 3 ? hp[v * SWX_T] : sS[(at[g] + v) * SWX_T];
+                if (AHEAD) return g == 2 ? hm[v * T] : g == 3 ? hp[v * T] : sS[(at[g] + v) * T];
                 return g < 2 ? own[6 * g + v] : __ldg(gp[g] + v * TILE3);
             };
             sweep_states<R, AMR, 0, OPT>(a, X, sq, dt, c, j, k, Vc, eb, e, vecL, vecR, sg, [] {}, Wm, Wp);
 #pragma unroll
-            for (int q = 0; q < 6; q++) sW[q * SWX_T + t] = Wp[q];
+            for (int q = 0; q < 6; q++) sW[q * T + t] = Wp[q];
             if (c >= f0 && c < N) {
                 R *w = X.wst[0] + G.widx(0, c, j, k);
                 w[0] = Wp[P];
@@ -566,7 +570,7 @@ __global__ void __launch_bounds__(SWX_T, SwxMinB<R>::value) sweepx3d_kernel(cons
         if (st && c >= f0) {
             R VL[6], F[NF];
 #pragma unroll
-            for (int q = 0; q < 6; q++) VL[q] = sW[q * SWX_T + t - 1];
+            for (int q = 0; q < 6; q++) VL[q] = sW[q * T + t - 1];
             const int er = riemann<R, 0, OPT>(a.prm, 0, VL, (R)V[GC * NWIN + wc - 1], (R)V[GE * NWIN + wc - 1], Wm,
                                          (R)V[GC * NWIN + wc], (R)V[GE * NWIN + wc], F);
             if (er) atomicOr(a.err, er);
@@ -575,43 +579,84 @@ __global__ void __launch_bounds__(SWX_T, SwxMinB<R>::value) sweepx3d_kernel(cons
     }
 }
 
-// The tile: of up to 16 lines per CTA the count with the fewest tiles per
-// plane, the line's faces split evenly over the segments.
-template <class R, int ORDER, bool AMR, int OPT> void launch_sweepx3d(const Args3D &a0, unsigned entries, cudaStream_t s)
+// The tile of a CTA of T threads: of up to 16 lines (no more than there are)
+// the count with the fewest tiles per plane, the line's faces split evenly
+// over the segments.
+template <class R, int ORDER, bool AMR, int T> SweepPlan plan_sweepx3d(Args3D &a, unsigned entries)
 {
-    Args3D a = a0;
     constexpr int EX = swx_extra<ORDER>();
-    long best = -1;
-    // (two lines at least where the tile's outer lines share rows of SWX_T values)
-    for (int t1 = swx_ahead<R>() ? 2 : 1; t1 <= 16; t1 *= 2) {
-        int len = SWX_T / t1 - EX;
+    long tiles = -1;
+    // (two lines at least where the tile's outer lines share rows of T values)
+    for (int t1 = swx_ahead<R>() ? 2 : 1; t1 <= 16 && (t1 <= 2 || t1 <= a.ny); t1++) {
+        int len = T / t1 - EX;
         len = len < a.nx + 1 ? len : a.nx + 1;
-        if (len < 2 || t1 * (len + 5) > 2 * SWX_T) continue;
+        if (len < 2 || t1 * (len + 5) > 2 * T) continue;
         const int segs = (a.nx + len) / len;
-        const long tiles = (long)segs * ((a.ny + t1 - 1) / t1);
-        if (best < 0 || tiles <= best) {
-            best = tiles;
+        const long n = (long)segs * ((a.ny + t1 - 1) / t1);
+        if (tiles < 0 || n <= tiles) {
+            tiles = n;
             a.swx_lines = t1;
             a.swx_segs = segs;
             a.swx_len = (a.nx + segs) / segs;
         }
     }
-    long chunks = cut_line(a.nz, FXB_SWX_PMIN, 1., best * entries, 148L * SwxMinB<R>::value);
+    const long resident = 148L * swx_resident<R, T>();
+    long chunks = cut_line(a.nz, FXB_SWX_PMIN, 1., tiles * entries, resident);
     a.swx_planes = (int)((a.nz + chunks - 1) / chunks);
     chunks = (a.nz + a.swx_planes - 1) / a.swx_planes;
     const size_t smem = 16 * (size_t)a.swx_lines * (a.swx_len + 5) * (AMR ? sizeof(R) : sizeof(double)) +
-                        ((ORDER == 3 ? 12 : 6) + (swx_ahead<R>() ? 30 : 0)) * (size_t)SWX_T * sizeof(R);
-    if (smem > 48 * 1024)
-        cudaFuncSetAttribute(sweepx3d_kernel<R, ORDER, AMR, OPT>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    sweepx3d_kernel<R, ORDER, AMR, OPT><<<dim3((unsigned)best, (unsigned)chunks, entries), SWX_T, smem, s>>>(a);
+                        ((ORDER == 3 ? 12 : 6) + (swx_ahead<R>() ? 30 : 0)) * (size_t)T * sizeof(R);
+    return {dim3((unsigned)tiles, (unsigned)chunks, entries), T, smem, (double)tiles * chunks * entries / resident};
 }
 
+// the plan of the sweep of direction DIR; its numbers into a
+template <class R, int ORDER, bool AMR, int DIR> SweepPlan plan_sweep3d(Args3D &a, unsigned entries)
+{
+    if constexpr (AMR) {
+        // the CTA size that leaves fewer threads of a leaf idle: us per step,
+        // 160 and 128 threads / the choice, 1,184 leaves of 8^3 PPM 654 / 623
+        // (FP32 340 / 317), WENO5 914 / 788 (374 / 338), 288 of 12^3 PPM 516 / 445
+        // (270 / 247).  FP32 keeps the larger where one piece of every
+        // line fills a quarter of the chip at most (64 leaves of 8^3: van Leer
+        // 45, 48 with the smaller).
+        Args3D b = a;
+        SweepPlan wide, narrow;
+        if constexpr (DIR == 0) {
+            wide = plan_sweepx3d<R, ORDER, AMR, 160>(a, entries);
+            narrow = plan_sweepx3d<R, ORDER, AMR, 96>(b, entries);
+        } else {
+            wide = plan_march3d<R, ORDER, DIR, 128>(a, entries);
+            narrow = plan_march3d<R, ORDER, DIR, 64>(b, entries);
+        }
+        if ((sizeof(R) == 4 && wide.waves <= 0.25 * wide.grid.y) ||
+            (long)narrow.threads * narrow.grid.x >= (long)wide.threads * wide.grid.x) return wide;
+        a = b;
+        return narrow;
+    } else if constexpr (DIR == 0) {
+        return plan_sweepx3d<R, ORDER, AMR, 160>(a, entries);
+    } else {
+        return plan_march3d<R, ORDER, DIR, 128>(a, entries);
+    }
+}
 // the sweep of direction DIR
 template <class R, int ORDER, bool AMR, int DIR, int OPT>
-void launch_sweep3d(const Args3D &a, unsigned entries, cudaStream_t s)
+void launch_sweep3d(const Args3D &a0, unsigned entries, cudaStream_t s)
 {
-    if constexpr (DIR == 0) launch_sweepx3d<R, ORDER, AMR, OPT>(a, entries, s);
-    else launch_march3d<R, ORDER, AMR, DIR, OPT>(a, entries, s);
+    Args3D a = a0;
+    const SweepPlan p = plan_sweep3d<R, ORDER, AMR, DIR>(a, entries);
+    auto go = [&](void (*k)(Args3D)) {
+        if (p.smem > 48 * 1024) cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)p.smem);
+        k<<<p.grid, p.threads, p.smem, s>>>(a);
+    };
+    if constexpr (DIR == 0) {
+        if constexpr (AMR)
+            if (p.threads == 96) return go(sweepx3d_kernel<R, ORDER, AMR, OPT, 96>);
+        go(sweepx3d_kernel<R, ORDER, AMR, OPT, 160>);
+    } else {
+        if constexpr (AMR)
+            if (p.threads == 64) return go(march3d_kernel<R, ORDER, AMR, DIR, OPT, 64>);
+        go(march3d_kernel<R, ORDER, AMR, DIR, OPT, 128>);
+    }
 }
 
 } // namespace fxb

@@ -103,28 +103,71 @@ def test_3d_sweep_extents_match_oracle(oracle, need_gpu, shape, order):
         _check(*_steps(oracle, geom, hp, S.noisy_gas(geom, hp)))
 
 
-@pytest.mark.parametrize("name", ["default", "vanLeer", "weno", "HLL"])
-def test_amr_option_matches_oracle(oracle, need_gpu, name):
-    geom = Geometry(3, 8, 8, 8, 2, 2, 2, bc=(BC_PERIODIC,) * 4 + (BC_REFLECTING,) * 2)
-    hp = dataclasses.replace(HydroParams(), **OPTIONS[name])
-    mesh, unk = A.levelset_problem(geom, hp, 2)
+def _amr(oracle, geom, hp, maxlev=2, n=2, precisions=("fp64", "mixed")):
+    """n steps of the level-set problem: (interiors per precision, oracle's, the last device's tuning text)."""
+    mesh, unk = A.levelset_problem(geom, hp, maxlev)
     am = oracle.Amr(oracle.make_params(geom.as_dict(), hp), mesh.levels, mesh.bcoords)
     dt = 0.4 * am.compute_dt(unk)
     ref = unk.copy()
-    for _ in range(2):
+    for _ in range(n):
         am.hydro_step(ref, dt)
     g = geom.nguard
     out = {}
-    for prec in ("fp64", "mixed"):
+    for prec in precisions:
         dev = HydroDevice(geom, hp, prec, mesh=mesh)
         dev.attach_unk(unk.copy())
-        for i in range(2):
+        for i in range(n):
             dev.Hydro(i * dt, dt, dt)
         o = unk.copy()
         dev.sync_to_host(o)
+        log = dev.tuning()
         dev.close()
         out[prec] = o[:, g:-g, g:-g, g:-g][..., HYDRO_VARS]
-    _check(out, ref[:, g:-g, g:-g, g:-g][..., HYDRO_VARS])
+    return out, ref[:, g:-g, g:-g, g:-g][..., HYDRO_VARS], log
+
+
+# both forms of the step, and every branch of the sweep kernels' boundary fluxes
+AMR_OPTIONS = {k: OPTIONS_3D[k] for k in ("default", "minmod", "vanLeer", "weno", "weno_HLL", "HLL", "no_ctu", "flattening",
+                                          "pressure_source")}
+
+
+@pytest.mark.parametrize("persistent", ["0", "1"])
+@pytest.mark.parametrize("name", sorted(AMR_OPTIONS))
+def test_amr_option_matches_oracle(oracle, need_gpu, monkeypatch, name, persistent):
+    monkeypatch.setenv("FXB_AMR_PERSISTENT", persistent)
+    geom = Geometry(3, 8, 8, 8, 2, 2, 2, bc=(BC_PERIODIC,) * 4 + (BC_REFLECTING,) * 2)
+    hp = dataclasses.replace(HydroParams(), **AMR_OPTIONS[name])
+    out, ref, log = _amr(oracle, geom, hp)
+    assert ("step form: persistent" if persistent == "1" else "step form: batched launches") in log
+    _check(out, ref)
+
+
+# leaves that fill the sweeps' CTAs of 64, 96, 128 and 160 threads and ones
+# that leave a remainder
+@pytest.mark.parametrize("order", [3, 5])
+@pytest.mark.parametrize("n", [4, 6, 8, 10, 12, 16])
+def test_amr_leaf_sizes_match_oracle(oracle, need_gpu, monkeypatch, n, order):
+    monkeypatch.setenv("FXB_AMR_PERSISTENT", "0")
+    geom = Geometry(3, n, n, n, 2, 1, 2, bc=(BC_PERIODIC,) * 2 + (BC_OUTFLOW,) * 2 + (BC_REFLECTING,) * 2)
+    _check(*_amr(oracle, geom, HydroParams(order=order))[:2])
+
+
+# more leaves than a batch takes: boundary fluxes stored in both passes; and
+# the smaller CTAs of FP32 leaves, which only larger batches take
+@pytest.mark.parametrize("opts", [{"slopeLimiter": "vanLeer"}, {"order": 5, "RiemannSolver": "HLL"},
+                                  {"hy_fPresInMomFlux": 0.5}])
+def test_amr_batches_of_sweeps_match_oracle(oracle, need_gpu, monkeypatch, opts):
+    monkeypatch.setenv("FXB_AMR_PERSISTENT", "0")
+    monkeypatch.setenv("FXB_AMR_MAX_BATCH", "23")
+    geom = Geometry(3, 8, 8, 8, 2, 2, 2, bc=(BC_PERIODIC,) * 6)
+    _check(*_amr(oracle, geom, dataclasses.replace(HydroParams(), **opts))[:2])
+
+
+@pytest.mark.parametrize("order", [3, 5])
+def test_amr_many_small_leaves_match_oracle(oracle, need_gpu, monkeypatch, order):
+    monkeypatch.setenv("FXB_AMR_PERSISTENT", "0")
+    geom = Geometry(3, 8, 8, 8, 3, 3, 3, bc=(BC_PERIODIC,) * 6)
+    _check(*_amr(oracle, geom, HydroParams(order=order), maxlev=3, n=1)[:2])
 
 
 # rows of whole 16-byte pairs, and (odd block sizes, odd slot counts) not;
