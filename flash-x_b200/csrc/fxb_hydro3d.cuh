@@ -1206,16 +1206,16 @@ template <class R> void set_pw_slots(Args3D &a, bool persistent = false)
 }
 
 // the rarely used options (Roe, contact steepening, MUSCL-Hancock) have kernel instantiations of their own
-template <class R, bool AMR, int DIR> void launch_states3d(const Args3D &a, dim3 g, cudaStream_t s)
+template <class R, bool AMR, int DIR> void launch_states3d(const Args3D &a, dim3 g, bool max_smem, cudaStream_t s)
 {
     if (!extended_options(a.prm)) {
         const bool o5 = a.prm.order == 5;
         if (default_options(a.prm)) {
-            if (o5) launch_sweep3d<R, 5, AMR, DIR, OPT_DEFAULT>(a, g.y, s);
-            else launch_sweep3d<R, 3, AMR, DIR, OPT_DEFAULT>(a, g.y, s);
+            if (o5) launch_sweep3d<R, 5, AMR, DIR, OPT_DEFAULT>(a, g.y, max_smem, s);
+            else launch_sweep3d<R, 3, AMR, DIR, OPT_DEFAULT>(a, g.y, max_smem, s);
         } else {
-            if (o5) launch_sweep3d<R, 5, AMR, DIR, OPT_ANY>(a, g.y, s);
-            else launch_sweep3d<R, 3, AMR, DIR, OPT_ANY>(a, g.y, s);
+            if (o5) launch_sweep3d<R, 5, AMR, DIR, OPT_ANY>(a, g.y, max_smem, s);
+            else launch_sweep3d<R, 3, AMR, DIR, OPT_ANY>(a, g.y, max_smem, s);
         }
         return;
     }
@@ -1231,6 +1231,14 @@ template <class R, bool AMR, int DIR> void launch_states3d(const Args3D &a, dim3
 // a large one's fill each other's last wave (136x88x120 0.855 -> 0.820 ms, PPM
 // 128^3 1.05 -> 1.04, mixed 0.59 -> 0.57, AMR 64 / 720 leaves of 16^3 222 -> 210 us
 // / 1.89 -> 1.87 ms).  The extended-option kernels share the slope array.
+//
+// CTAs of two kernels share an SM only under the same split of its memory
+// between L1 and shared memory, and the driver picks each kernel's.  Sweeps
+// that about fit on the chip together all ask for the largest shared memory
+// (FP32 PPM 32^3 42 -> 32 us per step, 40^3 49 -> 42, 32x48x40 48 -> 39; FP64 64
+// leaves of 8^3 62 -> 57); large ones keep the L1 they read sigma through (FP32
+// 128^3 563 us, 625 with the largest shared memory), and so do FP32 leaves
+// (64 of 8^3: van Leer 45 us, 48).
 struct SweepStreams {
     cudaStream_t side[2];
     cudaEvent_t fork, join[2];
@@ -1238,16 +1246,18 @@ struct SweepStreams {
 template <class R, bool AMR> void launch_sweeps3d(const Args3D &a, dim3 g, cudaStream_t s, const SweepStreams &st)
 {
     if (extended_options(a.prm)) {
-        launch_states3d<R, AMR, 0>(a, g, s);
-        launch_states3d<R, AMR, 1>(a, g, s);
-        launch_states3d<R, AMR, 2>(a, g, s);
+        launch_states3d<R, AMR, 0>(a, g, false, s);
+        launch_states3d<R, AMR, 1>(a, g, false, s);
+        launch_states3d<R, AMR, 2>(a, g, false, s);
         return;
     }
+    const bool max_smem = !(AMR && sizeof(R) == 4) &&
+                          (a.prm.order == 5 ? sweep_waves<R, 5, AMR>(a, g.y) : sweep_waves<R, 3, AMR>(a, g.y)) <= 1.5;
     cudaEventRecord(st.fork, s);
     for (int q = 0; q < 2; q++) cudaStreamWaitEvent(st.side[q], st.fork, 0);
-    launch_states3d<R, AMR, 0>(a, g, s);
-    launch_states3d<R, AMR, 1>(a, g, st.side[0]);
-    launch_states3d<R, AMR, 2>(a, g, st.side[1]);
+    launch_states3d<R, AMR, 0>(a, g, max_smem, s);
+    launch_states3d<R, AMR, 1>(a, g, max_smem, st.side[0]);
+    launch_states3d<R, AMR, 2>(a, g, max_smem, st.side[1]);
     for (int q = 0; q < 2; q++) {
         cudaEventRecord(st.join[q], st.side[q]);
         cudaStreamWaitEvent(s, st.join[q], 0);

@@ -638,15 +638,32 @@ template <class R, int ORDER, bool AMR, int DIR> SweepPlan plan_sweep3d(Args3D &
         return plan_march3d<R, ORDER, DIR, 128>(a, entries);
     }
 }
-// the sweep of direction DIR
+// chip fills of the three sweeps together
+template <class R, int ORDER, bool AMR> double sweep_waves(const Args3D &a0, unsigned entries)
+{
+    Args3D a = a0;
+    return plan_sweep3d<R, ORDER, AMR, 0>(a, entries).waves + plan_sweep3d<R, ORDER, AMR, 1>(a, entries).waves +
+           plan_sweep3d<R, ORDER, AMR, 2>(a, entries).waves;
+}
+// the sweep of direction DIR; max_smem: ask for the largest shared memory per SM
 template <class R, int ORDER, bool AMR, int DIR, int OPT>
-void launch_sweep3d(const Args3D &a0, unsigned entries, cudaStream_t s)
+void launch_sweep3d(const Args3D &a0, unsigned entries, bool max_smem, cudaStream_t s)
 {
     Args3D a = a0;
     const SweepPlan p = plan_sweep3d<R, ORDER, AMR, DIR>(a, entries);
     auto go = [&](void (*k)(Args3D)) {
         if (p.smem > 48 * 1024) cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)p.smem);
-        k<<<p.grid, p.threads, p.smem, s>>>(a);
+        cudaLaunchAttribute at{};
+        at.id = cudaLaunchAttributePreferredSharedMemoryCarveout;
+        at.val.sharedMemCarveout = cudaSharedmemCarveoutMaxShared;
+        cudaLaunchConfig_t c{};
+        c.gridDim = p.grid;
+        c.blockDim = dim3(p.threads);
+        c.dynamicSmemBytes = p.smem;
+        c.stream = s;
+        c.attrs = &at;
+        c.numAttrs = max_smem ? 1 : 0;
+        cudaLaunchKernelEx(&c, k, a);
     };
     if constexpr (DIR == 0) {
         if constexpr (AMR)
