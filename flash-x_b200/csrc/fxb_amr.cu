@@ -94,6 +94,7 @@ struct State {
     std::vector<long> rlist_off;                  // per level offset into d_rlist, size maxlev + 1
     int cta[4] = {4, 4, 4, 4};                    // CTAs per block: sig, slopes, (unused), update
     int fill_cta = 8;
+    bool stages = true;                           // FP64 WENO5: per-stage kernels (until amr_tune times both forms)
     bool tuned = false;                           // launch shapes chosen (first attach of the mesh)
     char tune_log[512] = "";
     std::unordered_map<uint64_t, int> map;
@@ -843,6 +844,7 @@ Args3D batch_args(const double *dtv, double dt)
     a.istore = S.store[S.cur];
     a.dxl = S.d_dxl;
     for (int q = 0; q < 4; q++) a.cta[q] = S.cta[q];
+    a.stages = S.stages;
     a.odata = S.store[1 - S.cur]; a.o_vstride = S.vstride; a.o_bstride = S.bstride;
     a.bflux = S.bflux;
     a.nfc = S.nfc;
@@ -1386,10 +1388,11 @@ int batched_step(const double *dtv, double dt, int &nl)
         if (mixed) launch_amr3d_fluxes_mixed(a, cnt, all, S.C.stream, S.C.sweeps);
         else launch_amr3d_fluxes_fp64(a, cnt, all, S.C.stream, S.C.sweeps);
     };
-    // the default options' sweeps store the boundary fluxes themselves
-    const bool ext = extended_options(S.C.dprm);
+    // the sweep kernels store the boundary fluxes themselves
+    const SweepForm form = mixed ? hydro3d_form_mixed(a) : hydro3d_form_fp64(a);
     auto emit = [&](int cnt) {
-        if (!ext) return;
+        if (form == SWEEP_KERNELS) return;
+        nl++;
         if (mixed) launch_amr3d_emit_mixed(a, cnt, S.bflux, S.nfc, S.C.stream);
         else launch_amr3d_emit_fp64(a, cnt, S.bflux, S.nfc, S.C.stream);
     };
@@ -1401,21 +1404,21 @@ int batched_step(const double *dtv, double dt, int &nl)
         if (mixed) launch_amr3d_update_mixed(a, cnt, S.C.stream); else launch_amr3d_update_fp64(a, cnt, S.C.stream);
     };
     // sigma (+ flattening), then per direction the slopes, face states and
-    // fluxes (one kernel; with extended options in FP64 slopes (PPM), face
-    // states and fluxes as separate kernels)
-    const int pipe = 1 + (S.C.prm.flattening ? 1 : 0) + 3 * (mixed || !ext ? 1 : (S.C.prm.order == 3 ? 3 : 2));
+    // fluxes (one kernel, or slopes (PPM), face states and fluxes as separate
+    // kernels)
+    const int pipe = 1 + (S.C.prm.flattening ? 1 : 0) + 3 * (form != STAGE_KERNELS ? 1 : (S.C.prm.order == 3 ? 3 : 2));
     if (S.nstep <= S.batch) {
         a.batch = S.d_step_entries;
         nl += fill_batch(a.batch, S.nstep, S.cur);
         fluxes(S.nstep); emit(S.nstep); correct(S.nstep); update(S.nstep);
-        nl += pipe + 2 + ext;
+        nl += pipe + 2;
     } else {
         for (int l0 = 0; l0 < S.nstep; l0 += S.batch) {
             int cnt = std::min(S.batch, S.nstep - l0);
             a.batch = S.d_step_entries + S.nstep + l0;
             nl += fill_batch(a.batch, cnt, S.cur);
             fluxes(cnt); emit(cnt); update(cnt);
-            nl += pipe + 1 + ext;
+            nl += pipe + 1;
         }
         for (int l0 = 0; l0 < S.nstep_finer; l0 += S.batch) {
             int cnt = std::min(S.batch, S.nstep_finer - l0);
@@ -1429,16 +1432,19 @@ int batched_step(const double *dtv, double dt, int &nl)
     return FXB_OK;
 }
 
-// Launch-shape search on the attached state: the guard fill, sigma, the PPM
-// slopes and the update are timed with 1, 2, 4, 8 and 16 CTAs per block (one
-// warm-up pass, one timed pass each) and the fastest count per stage is kept
-// (the face-state and flux kernel has fixed tiles and is timed with the
-// slopes).  The stages compute cells independently, so the choice changes
+// Launch-shape search on the attached state: the guard fill, sigma, where they
+// run the per-stage kernels' CTAs (timed with the fluxes), and the update are
+// timed with 1, 2, 4, 8 and 16 CTAs per block (one warm-up pass, one timed pass
+// each) and the fastest count per stage is kept; then whole steps in the forms
+// there are (FP64 WENO5: sweep kernels against per-stage ones; the persistent
+// kernel).  The stages compute cells independently, so the counts change
 // timings, never results.  The update writes the other interior store, which
 // the next step overwrites.
 int amr_tune()
 {
-    const char *ev = getenv("FXB_AMR_TUNE");
+    const char *ev = getenv("FXB_AMR_TUNE"), *es = getenv("FXB_WENO_STAGES");
+    const bool choice = sweep_choice(S.C.dprm, S.C.prm.precision == FXB_FP64);
+    if (choice && es) S.stages = es[0] == '1';
     if (ev && atoi(ev) == 0) {
         snprintf(S.tune_log, sizeof(S.tune_log), "AMR launch shape (CTAs per block): fill=%d sig=%d slopes=%d "
                  "update=%d, defaults (tuning off); step form: %s", S.fill_cta, S.cta[0], S.cta[1], S.cta[3],
@@ -1453,53 +1459,85 @@ int amr_tune()
     float best[4] = {1e30f, 1e30f, 1e30f, 1e30f};
     int pick[4] = {S.fill_cta, S.cta[0], S.cta[1], S.cta[3]};
     restrict_all(S.cur);
-    for (int c : cand) {
-        S.fill_cta = c;
-        for (int q = 0; q < 4; q++) S.cta[q] = c;
-        Args3D a = batch_args(nullptr, 0.0);
-        a.batch = S.d_entries;
-        float t[4] = {0, 0, 0, 0};
-        for (int rep = 0; rep < 2; rep++) {
-            CKA(cudaEventRecord(e[0], S.C.stream));
-            fill_batch(a.batch, cnt, S.cur);
-            CKA(cudaEventRecord(e[1], S.C.stream));
-            for (int st = 0; st < 2; st++) {
-                if (mixed) launch_amr3d_fluxes_mixed(a, cnt, 1 << st, S.C.stream, S.C.sweeps);
-                else launch_amr3d_fluxes_fp64(a, cnt, 1 << st, S.C.stream, S.C.sweeps);
-                CKA(cudaEventRecord(e[2 + st], S.C.stream));
+    auto search = [&]() -> int {
+        // (the sweep and tile kernels choose their own grids)
+        const bool counts = !mixed && hydro3d_form_fp64(batch_args(nullptr, 0.0)) == STAGE_KERNELS;
+        for (float &b : best) b = 1e30f;
+        for (int c : cand) {
+            S.fill_cta = c;
+            for (int q = 0; q < 4; q++) S.cta[q] = c;
+            Args3D a = batch_args(nullptr, 0.0);
+            a.batch = S.d_entries;
+            float t[4] = {0, 0, 0, 0};
+            for (int rep = 0; rep < 2; rep++) {
+                CKA(cudaEventRecord(e[0], S.C.stream));
+                fill_batch(a.batch, cnt, S.cur);
+                CKA(cudaEventRecord(e[1], S.C.stream));
+                for (int st = 0; st < 2; st++) {
+                    if (mixed) launch_amr3d_fluxes_mixed(a, cnt, 1 << st, S.C.stream, S.C.sweeps);
+                    else launch_amr3d_fluxes_fp64(a, cnt, 1 << st, S.C.stream, S.C.sweeps);
+                    CKA(cudaEventRecord(e[2 + st], S.C.stream));
+                }
+                if (mixed) launch_amr3d_update_mixed(a, cnt, S.C.stream); else launch_amr3d_update_fp64(a, cnt, S.C.stream);
+                CKA(cudaEventRecord(e[4], S.C.stream));
+                CKA(cudaGetLastError());
+                CKA(cudaEventSynchronize(e[4]));
+                for (int k = 0; k < 4; k++) CKA(cudaEventElapsedTime(&t[k], e[k], e[k + 1]));
             }
-            if (mixed) launch_amr3d_update_mixed(a, cnt, S.C.stream); else launch_amr3d_update_fp64(a, cnt, S.C.stream);
-            CKA(cudaEventRecord(e[4], S.C.stream));
-            CKA(cudaGetLastError());
-            CKA(cudaEventSynchronize(e[4]));
-            for (int k = 0; k < 4; k++) CKA(cudaEventElapsedTime(&t[k], e[k], e[k + 1]));
+            for (int k = 0; k < 4; k++)
+                if (t[k] < best[k]) { best[k] = t[k]; pick[k] = c; }
         }
-        for (int k = 0; k < 4; k++)
-            if (t[k] < best[k]) { best[k] = t[k]; pick[k] = c; }
-    }
-    S.fill_cta = pick[0];
-    S.cta[0] = pick[1];
-    S.cta[1] = pick[2];
-    S.cta[2] = pick[2];
-    S.cta[3] = pick[3];
+        if (!counts) pick[2] = 4;
+        S.fill_cta = pick[0];
+        S.cta[0] = pick[1];
+        S.cta[1] = pick[2];
+        S.cta[2] = pick[2];
+        S.cta[3] = pick[3];
+        return FXB_OK;
+    };
+    int src = search();
+    if (src) return src;
     // the step's form: one persistent kernel with clusters of K CTAs per
     // leaf, or the batched launches; each timed over a whole step (one
     // warm-up run, one timed run), the fastest kept.  FXB_AMR_PERSISTENT=1
     // keeps the persistent kernel, FXB_AMR_CLUSTER=K its cluster size.
-    char form[160] = "";
-    if (S.persist_ok && !S.test_stall) {
-        auto time_step = [&](bool pers, float &ms) -> int {
-            for (int rep = 0; rep < 2; rep++) {
-                CKA(cudaEventRecord(e[0], S.C.stream));
+    char form[160] = "", sweeps[128] = "";
+    auto time_step = [&](bool pers, float &ms, int steps = 1) -> int {
+        for (int rep = 0; rep < 2; rep++) {
+            CKA(cudaEventRecord(e[0], S.C.stream));
+            for (int q = 0; q < steps; q++) {
                 int nl = 0;
                 int rc = pers ? persist_step(nullptr, 0.0) : batched_step(nullptr, 0.0, nl);
                 if (rc) return rc;
-                CKA(cudaEventRecord(e[1], S.C.stream));
-                CKA(cudaEventSynchronize(e[1]));
-                CKA(cudaEventElapsedTime(&ms, e[0], e[1]));
             }
-            return FXB_OK;
-        };
+            CKA(cudaEventRecord(e[1], S.C.stream));
+            CKA(cudaEventSynchronize(e[1]));
+            CKA(cudaEventElapsedTime(&ms, e[0], e[1]));
+        }
+        ms /= steps;
+        return FXB_OK;
+    };
+    if (choice && !es) {
+        // the best of three: sweep kernels, per-stage kernels; several steps in
+        // a row, or the forms' different numbers of launches count on a small mesh
+        float t[2] = {1e30f, 1e30f};
+        for (int rep = 0; rep < 3; rep++)
+            for (int st = 0; st < 2; st++) {
+                S.stages = st == 1;
+                float ms = 0.f;
+                int rc = time_step(false, ms, 4);
+                if (rc) return rc;
+                t[st] = std::min(t[st], ms);
+            }
+        S.stages = t[1] < t[0];
+        if (!S.stages) {
+            src = search();
+            if (src) return src;
+        }
+        snprintf(sweeps, sizeof(sweeps), "; sweeps: %s (ms per step: sweep kernels %.3f, per stage %.3f)",
+                 S.stages ? "per-stage kernels" : "one kernel per direction", t[0], t[1]);
+    }
+    if (S.persist_ok && !S.test_stall) {
         float tb = 0.f;
         int rc = time_step(false, tb);
         if (rc) return rc;
@@ -1531,8 +1569,8 @@ int amr_tune()
     CKA(cudaStreamSynchronize(S.C.stream));
     snprintf(S.tune_log, sizeof(S.tune_log),
              "AMR launch shape (CTAs of 256 per block, %d blocks of %d^3): fill=%d sig=%d slopes=%d update=%d "
-             "(ms fill %.3f, sigma %.3f, slopes + face states + fluxes %.3f, update %.3f)%s", cnt, S.n, pick[0],
-             pick[1], pick[2], pick[3], best[0], best[1], best[2], best[3], form);
+             "(ms fill %.3f, sigma %.3f, slopes + face states + fluxes %.3f, update %.3f)%s%s", cnt, S.n, pick[0],
+             pick[1], pick[2], pick[3], best[0], best[1], best[2], best[3], sweeps, form);
     return FXB_OK;
 }
 
@@ -1676,6 +1714,7 @@ int amr_regrid(const fxb_block_desc *leaves, int nleaf)
         cudaFree(ostore);
         S.fill_cta = old.fill_cta;
         for (int q = 0; q < 4; q++) S.cta[q] = old.cta[q];
+        S.stages = old.stages;
         snprintf(S.tune_log, sizeof(S.tune_log), "%s", old.tune_log);
         S.tuned = old.tuned;
         return code;
@@ -1732,6 +1771,7 @@ int amr_regrid(const fxb_block_desc *leaves, int nleaf)
     // size; the shapes change timings, never results)
     S.fill_cta = old.fill_cta;
     for (int q = 0; q < 4; q++) S.cta[q] = old.cta[q];
+    S.stages = old.stages;
     snprintf(S.tune_log, sizeof(S.tune_log), "%s", old.tune_log);
     S.tuned = old.tuned;
     return rc;

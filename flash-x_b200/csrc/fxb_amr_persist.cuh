@@ -321,7 +321,7 @@ template <class R> cudaError_t persist_upload_t(const PersistArgs p0[2])
     PersistArgs p[2] = {p0[0], p0[1]};
     for (int w = 0; w < 2; w++) {
         p[w].a = with_divisors(p0[w].a, sflux_halo<R>(p0[w].a));
-        set_pw_slots<R>(p[w].a, true);
+        set_pw_slots<R>(p[w].a, FusedFaces<R>::value ? FUSED_TILES : STAGE_KERNELS);
     }
     return cudaMemcpyToSymbol(c_persist_raw, p, sizeof(p));
 }

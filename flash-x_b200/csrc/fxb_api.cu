@@ -105,6 +105,7 @@ struct Lib {
     int use_tma = 1;
     // launch shapes of the uniform grid, chosen by ug_tune at the first attach
     bool ug_tuned = false;
+    bool stages = true;            // FP64 WENO5 in 3-D: per-stage kernels (until ug_tune times both forms)
     int ug_cta[4] = {8, 8, 8, 8};  // 3-D: CTAs per SM of sigma, face states, fluxes, update
     int sf_t1[3] = {0, 0, 0};      // 3-D FP32: lines per fused face-state tile (0: by lane count)
     char ug_log[512] = "";
@@ -483,6 +484,39 @@ int encode_window_map(CUtensorMap *m, const double *base)
 
 int launch_species(int src, const double *dtv, double dt);
 
+// the arguments of one 3-D step reading buffer `src`, writing 1-src
+Args3D ug_args3d(int src, const double *dtv, double dt)
+{
+    Args3D a;
+    a.in = L.buf[src]; a.out = L.buf[1 - src]; a.vstride = L.vstride;
+    a.nx = L.nx; a.ny = L.ny; a.nz = L.nz;
+    for (int i = 0; i < 6; i++) a.bc[i] = L.kbc[i];
+    a.rate_c0 = (long)L.slab.halo_lo * L.plane;
+    a.rate_c1 = a.rate_c0 + (long)L.nint * L.plane;
+    a.dx = cell_dx(0); a.dy = cell_dx(1); a.dz = cell_dx(2);
+    a.dt_arg = dt; a.dtv = dtv;
+    a.gam1inv = L.gam1inv; a.ggprodinv = L.ggprodinv;
+    a.prm = L.dprm; a.rate_max = L.rate_max; a.err = L.err;
+    a.sig = L.sig3;
+    a.slp = L.slp3;
+    a.slp_bstride = 0;
+    a.flat = L.flat;
+    a.flat_bstride = 0;
+    a.hyb = (const unsigned char *)L.hyb;
+    for (int d = 0; d < 3; d++) { a.wst[d] = L.w3[d]; a.flx[d] = L.f3[d]; a.ctufb[d] = L.ctufb[d]; }
+    for (int q = 0; q < 4; q++) a.cta[q] = 148 * L.ug_cta[q];
+    a.shok = L.shok;
+    for (int d = 0; d < 3; d++) a.sf_t1[d] = L.sf_t1[d];
+    a.stages = L.stages;
+    return a;
+}
+// the kernels the 3-D step's sweeps run as
+SweepForm ug_form()
+{
+    const Args3D a = ug_args3d(L.cur, nullptr, 0.);
+    return L.prm.precision == FXB_MIXED ? hydro3d_form_mixed(a) : hydro3d_form_fp64(a);
+}
+
 // launch one fused hydro step reading buffer `src`, writing 1-src
 int launch_hydro(int src, const double *dtv, double dt)
 {
@@ -513,26 +547,7 @@ int launch_hydro(int src, const double *dtv, double dt)
         if (L.prm.precision == FXB_MIXED) launch_hydro2d_mixed(a, grid, L.stream);
         else launch_hydro2d_fp64(a, grid, L.stream);
     } else {
-        Args3D a;
-        a.in = L.buf[src]; a.out = L.buf[1 - src]; a.vstride = L.vstride;
-        a.nx = L.nx; a.ny = L.ny; a.nz = L.nz;
-        for (int i = 0; i < 6; i++) a.bc[i] = L.kbc[i];
-        a.rate_c0 = (long)L.slab.halo_lo * L.plane;
-        a.rate_c1 = a.rate_c0 + (long)L.nint * L.plane;
-        a.dx = cell_dx(0); a.dy = cell_dx(1); a.dz = cell_dx(2);
-        a.dt_arg = dt; a.dtv = dtv;
-        a.gam1inv = L.gam1inv; a.ggprodinv = L.ggprodinv;
-        a.prm = L.dprm; a.rate_max = L.rate_max; a.err = L.err;
-        a.sig = L.sig3;
-        a.slp = L.slp3;
-        a.slp_bstride = 0;
-        a.flat = L.flat;
-        a.flat_bstride = 0;
-        a.hyb = (const unsigned char *)L.hyb;
-        for (int d = 0; d < 3; d++) { a.wst[d] = L.w3[d]; a.flx[d] = L.f3[d]; a.ctufb[d] = L.ctufb[d]; }
-        for (int q = 0; q < 4; q++) a.cta[q] = 148 * L.ug_cta[q];
-        a.shok = L.shok;
-        for (int d = 0; d < 3; d++) a.sf_t1[d] = L.sf_t1[d];
+        const Args3D a = ug_args3d(src, dtv, dt);
         for (int d = 0; d < 3 && L.ns; d++)
             if (cudaMemsetAsync(L.ctufb[d], 0, L.snw, L.stream) != cudaSuccess) return cuda_fail(cudaGetLastError(), "memset");
         if (L.prm.precision == FXB_MIXED) launch_hydro3d_mixed(a, L.stream, L.sweeps);
@@ -573,17 +588,17 @@ int launch_species(int src, const double *dtv, double dt)
 }
 
 // kernels of one 3-D step: sigma, per direction the slopes, face states and
-// fluxes (one kernel; with extended options in FP64 slopes (PPM), face states
-// and fluxes as separate kernels), the update
-int hydro3d_launches(const fxb_params &p)
+// fluxes (one kernel, or slopes (PPM), face states and fluxes as separate
+// kernels), the update
+int hydro3d_launches()
 {
-    const int per_dir = p.precision == FXB_MIXED || !extended_options(L.dprm) ? 1 : (p.order == 3 ? 3 : 2);
+    const int per_dir = ug_form() != STAGE_KERNELS ? 1 : (L.prm.order == 3 ? 3 : 2);
     return 1 + 3 * per_dir + 1;
 }
 // launches of one uniform-grid step (flattening and species add kernels)
 int ug_step_launches()
 {
-    return (L.dom.ndim == 2 ? 1 : hydro3d_launches(L.prm)) + (L.prm.flattening ? 1 : 0) + (L.ns ? 3 : 0);
+    return (L.dom.ndim == 2 ? 1 : hydro3d_launches()) + (L.prm.flattening ? 1 : 0) + (L.ns ? 3 : 0);
 }
 
 // the step's scalars into the page-locked record, after the stream's work
@@ -966,19 +981,21 @@ extern "C" int fxb_register_blocks(const fxb_block_desc *blocks, int nblk)
 }
 
 // one step from the current state with dt = 0 (the state is not switched):
-// the fastest of `reps` runs, in ms
-static int time_ug_step(float &best, int reps)
+// the fastest of `reps` runs of `steps` steps each, in ms per step
+static int time_ug_step(float &best, int reps, int steps = 1)
 {
     best = 1e30f;
     for (int r = 0; r < reps; r++) {
         CK(cudaEventRecord(L.ev0, L.stream));
-        int rc = launch_hydro(L.cur, nullptr, 0.0);
-        if (rc) return rc;
+        for (int q = 0; q < steps; q++) {
+            int rc = launch_hydro(L.cur, nullptr, 0.0);
+            if (rc) return rc;
+        }
         CK(cudaEventRecord(L.ev1, L.stream));
         CK(cudaEventSynchronize(L.ev1));
         float ms = 0.f;
         CK(cudaEventElapsedTime(&ms, L.ev0, L.ev1));
-        best = ms < best ? ms : best;
+        best = ms / steps < best ? ms / steps : best;
     }
     return FXB_OK;
 }
@@ -986,14 +1003,19 @@ static int time_ug_step(float &best, int reps)
 // The uniform grid's launch shapes, timed over whole steps on the attached
 // state at the first attach: 2-D window staging by TMA or by per-thread
 // loads; 3-D CTAs per SM of each stage (2, 4, 8, 16), one stage at a time,
-// and in FP32 the lines per fused face-state tile of each direction.  A
+// in FP32 the lines per fused face-state tile of each direction, and for FP64
+// WENO5 the sweep kernels against the per-stage ones (sweep_form).  A
 // candidate replaces the current choice when it is more than 1 % faster.
-// FXB_UG_TUNE=0 keeps the defaults; FXB_TMA=0/1 fixes the 2-D staging.  The
+// FXB_UG_TUNE=0 keeps the defaults; FXB_TMA=0/1 fixes the 2-D staging,
+// FXB_WENO_STAGES=0/1 the kernels.  The
 // timed steps leave no trace: the CFL rate and the error word are cleared.
 static int ug_tune()
 {
     const char *ev = getenv("FXB_UG_TUNE");
     const bool off = ev && ev[0] == '0';
+    const char *es = getenv("FXB_WENO_STAGES");
+    const bool choice = L.dom.ndim == 3 && sweep_choice(L.dprm, L.prm.precision == FXB_FP64);
+    if (choice && es) L.stages = es[0] == '1';
     float base = 0.f;
     int rc = FXB_OK;
     if (!off) {
@@ -1020,8 +1042,6 @@ static int ug_tune()
                  "staging: %s (ms per step: TMA %.3f, per-thread loads %.3f%s)", L.use_tma ? "TMA" : "per-thread loads",
                  t[1], t[0], off ? ", tuning off" : "");
     } else {
-        // the default options' sweeps choose their own grids
-        const bool fused = L.prm.precision == FXB_MIXED, ext = extended_options(L.dprm);
         float cur = base;
         // FXB_UG_CTA="s,f,x,u" and FXB_UG_T1="x,y,z" fix the shapes instead
         const char *ec = getenv("FXB_UG_CTA"), *et = getenv("FXB_UG_T1");
@@ -1037,22 +1057,42 @@ static int ug_tune()
                 return fail(FXB_EARG, "FXB_UG_T1: three line counts expected");
             for (int d = 0; d < 3; d++) L.sf_t1[d] = v[d] < 0 ? 0 : v[d];
         }
-        if (!off && !ec && !et) {
-            const int cand[4] = {2, 4, 8, 16};
-            for (int q = 0; q < 4; q++) {
-                if ((fused || !ext) && (q == 1 || q == 2)) continue;     // the fused kernel's grid follows its tiles
-                int keep = L.ug_cta[q];
-                for (int c : cand) {
-                    if (c == keep) continue;
-                    L.ug_cta[q] = c;
-                    float t = 0.f;
-                    rc = time_ug_step(t, 3);
-                    if (rc) return rc;
-                    if (t < 0.99f * cur) { cur = t; keep = c; }
-                    L.ug_cta[q] = keep;
-                }
+        auto tune_cta = [&](int q) -> int {
+            int keep = L.ug_cta[q];
+            for (int c : {2, 4, 8, 16}) {
+                if (c == keep) continue;
+                L.ug_cta[q] = c;
+                float t = 0.f;
+                int trc = time_ug_step(t, 3);
+                if (trc) return trc;
+                if (t < 0.99f * cur) { cur = t; keep = c; }
+                L.ug_cta[q] = keep;
             }
-            if (fused && ext)
+            return FXB_OK;
+        };
+        if (!off && !ec && !et) {
+            // the per-stage kernels' counts (the sweep and tile kernels choose their own grids)
+            for (int q = 1; q < 3 && !rc && ug_form() == STAGE_KERNELS; q++) rc = tune_cta(q);
+            if (rc) return rc;
+        }
+        if (!off && choice && !es) {
+            // several steps in a row, or the forms' different numbers of
+            // launches count on a small grid
+            float t[2] = {0.f, 0.f};
+            for (int st = 1; st >= 0 && !rc; st--) {
+                L.stages = st == 1;
+                rc = time_ug_step(t[st], 3, 6);
+            }
+            if (rc) return rc;
+            L.stages = t[1] < t[0];
+            rc = time_ug_step(cur, 3);
+            if (rc) return rc;
+        }
+        const SweepForm form = ug_form();
+        if (!off && !ec && !et) {
+            for (int q = 0; q < 4 && !rc; q += 3) rc = tune_cta(q);
+            if (rc) return rc;
+            if (form == FUSED_TILES)
                 for (int d = 0; d < 3; d++) {
                     int keep = L.sf_t1[d];
                     for (int t1 : {1, 2, 4, 8, 16}) {
@@ -1066,11 +1106,11 @@ static int ug_tune()
                 }
         }
         char tiles[96] = "";
-        if (fused) snprintf(tiles, sizeof(tiles), "; face-state tile lines x/y/z: %d/%d/%d (0: by lane count)",
+        if (L.prm.precision == FXB_MIXED) snprintf(tiles, sizeof(tiles), "; face-state tile lines x/y/z: %d/%d/%d (0: by lane count)",
                             L.sf_t1[0], L.sf_t1[1], L.sf_t1[2]);
         snprintf(L.ug_log, sizeof(L.ug_log), "uniform grid 3-D: CTAs of 256 threads per SM: sigma %d, face states %d, "
-                 "fluxes %d, update %d%s (ms per step: defaults %.3f, tuned %.3f%s)", L.ug_cta[0], L.ug_cta[1],
-                 L.ug_cta[2], L.ug_cta[3], tiles, base, cur, off ? ", tuning off" : "");
+                 "fluxes %d, update %d%s; sweeps: %s (ms per step: defaults %.3f, tuned %.3f%s)", L.ug_cta[0], L.ug_cta[1],
+                 L.ug_cta[2], L.ug_cta[3], tiles, sweep_form_name(form), base, cur, off ? ", tuning off" : "");
     }
     CK(cudaMemsetAsync(L.rate_max, 0, sizeof(unsigned long long), L.stream));
     CK(cudaMemsetAsync(L.err, 0, sizeof(int), L.stream));

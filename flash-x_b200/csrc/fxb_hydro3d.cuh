@@ -94,6 +94,7 @@ struct Args3D {
     long nfc = 0;
     unsigned char *ctufb[3] = {nullptr, nullptr, nullptr};   // species on: 1 where the CTU fallback fired (Grid3::widx)
     const unsigned char *shok = nullptr;   // shock detector on (uniform grid): the flag of every cell
+    int stages = 0;             // FP64 WENO5: per-stage kernels instead of the sweep kernels (sweep_form)
 };
 // Face-state tile of direction d (N cells along d, N1 along the t1 axis):
 // the fewest warp lanes in total (the N + 1 faces split into segments of
@@ -1174,7 +1175,7 @@ template <class R, bool AMR, int DIR, int EXT> void launch_states3d_rs(const Arg
         constexpr int SX = EXT ? 1 : 0;
         if (a.prm.order == 5) {
             states3d_kernel<R, 5, AMR, DIR, SX><<<g, 256, 0, s>>>(a);
-        } else {
+        } else if constexpr (EXT) {            // (PPM with the default options: the sweep kernels)
             slope3d_kernel<R, AMR><<<g, 256, 0, s>>>(a, DIR);
             states3d_kernel<R, 3, AMR, DIR, SX><<<g, 256, 0, s>>>(a);
         }
@@ -1193,44 +1194,66 @@ template <class R, bool AMR, int DIR, int EXT> void launch_states3d_rs(const Arg
         }
     }
 }
-// whether a direction of a step with these options runs as one kernel that
-// stores the fluxes and the two face pressures only
-template <class R> bool one_kernel_sweep(const DevParams &p) { return FusedFaces<R>::value || !extended_options(p); }
-template <class R> void set_pw_slots(Args3D &a, bool persistent = false)
+// The kernels of the three sweeps: one per direction (fxb_march3d.cuh), or with
+// extended options the fused tile kernel (FP32) or slopes, face states and
+// fluxes as separate kernels (FP64).  FP64 WENO5 may take the separate kernels
+// with the other options too (Args3D::stages).  Neither form is the faster one
+// everywhere: the per-stage kernels keep 16 warps per SM on the long WENO chain
+// and leave no last wave, the sweeps run side by side and move less.  us per
+// step, sweeps / per stage: 32^3 58 / 68, 40^3 89 / 70, 64^3 225 / 228, 80^3
+// 425 / 405, 112^3 1009 / 1037, 128^3 1498 / 1505, 80^3 with HLL 465 / 405; AMR, 16
+// leaves of 16^3 97 / 122, 288 of 16^3 1106 / 1095, 64 of 12^3 177 / 146, 288 of
+// 12^3 590 / 541.  The tuners time both on the attached state (fxb_api.cu,
+// fxb_amr.cu); the results are the same bits.
+enum SweepForm { SWEEP_KERNELS, FUSED_TILES, STAGE_KERNELS };
+// whether a step with these options has the choice
+__host__ __device__ inline bool sweep_choice(const DevParams &p, bool fp64) { return fp64 && p.order == 5 && !extended_options(p); }
+template <class R> SweepForm sweep_form(const Args3D &a)
+{
+    if (!extended_options(a.prm) && !(sweep_choice(a.prm, sizeof(R) == 8) && a.stages)) return SWEEP_KERNELS;
+    return FusedFaces<R>::value ? FUSED_TILES : STAGE_KERNELS;
+}
+inline const char *sweep_form_name(SweepForm f)
+{
+    return f == SWEEP_KERNELS ? "one kernel per direction with its own grid"
+           : f == FUSED_TILES ? "fused face-state tiles" : "per-stage kernels";
+}
+template <class R> void set_pw_slots(Args3D &a, SweepForm form)
 {
     for (int d = 0; d < 3; d++) {
-        const PwSlots q = pw_slots<R>(!persistent && one_kernel_sweep<R>(a.prm));
+        const PwSlots q = pw_slots<R>(form != STAGE_KERNELS);
         a.pw_wp[d] = q.wp;
         a.pw_wm[d] = q.wm;
     }
 }
 
-// the rarely used options (Roe, contact steepening, MUSCL-Hancock) have kernel instantiations of their own
-template <class R, bool AMR, int DIR> void launch_states3d(const Args3D &a, dim3 g, bool max_smem, cudaStream_t s)
+// one direction as per-stage kernels; the rarely used options (Roe, contact
+// steepening, MUSCL-Hancock) and the Marquina solvers have instantiations of their own
+template <class R, bool AMR, int DIR> void launch_stages3d(const Args3D &a, dim3 g, cudaStream_t s)
 {
-    if (!extended_options(a.prm)) {
-        const bool o5 = a.prm.order == 5;
-        if (default_options(a.prm)) {
-            if (o5) launch_sweep3d<R, 5, AMR, DIR, OPT_DEFAULT>(a, g.y, max_smem, s);
-            else launch_sweep3d<R, 3, AMR, DIR, OPT_DEFAULT>(a, g.y, max_smem, s);
-        } else {
-            if (o5) launch_sweep3d<R, 5, AMR, DIR, OPT_ANY>(a, g.y, max_smem, s);
-            else launch_sweep3d<R, 3, AMR, DIR, OPT_ANY>(a, g.y, max_smem, s);
-        }
-        return;
-    }
     if (marquina_solver(a.prm)) launch_states3d_rs<R, AMR, DIR, 2>(a, g, s);
     else if (extended_options(a.prm)) launch_states3d_rs<R, AMR, DIR, 1>(a, g, s);
-    else launch_states3d_rs<R, AMR, DIR, 0>(a, g, s);
+    else if constexpr (sizeof(R) == 8) launch_states3d_rs<R, AMR, DIR, 0>(a, g, s);
+}
+template <class R, bool AMR, int DIR> void launch_one_sweep3d(const Args3D &a, unsigned entries, bool max_smem, cudaStream_t s)
+{
+    const bool o5 = a.prm.order == 5;
+    if (default_options(a.prm)) {
+        if (o5) launch_sweep3d<R, 5, AMR, DIR, OPT_DEFAULT>(a, entries, max_smem, s);
+        else launch_sweep3d<R, 3, AMR, DIR, OPT_DEFAULT>(a, entries, max_smem, s);
+    } else {
+        if (o5) launch_sweep3d<R, 5, AMR, DIR, OPT_ANY>(a, entries, max_smem, s);
+        else launch_sweep3d<R, 3, AMR, DIR, OPT_ANY>(a, entries, max_smem, s);
+    }
 }
 
-// The three sweeps of a step.  With the default options they share only what
-// they read (state and sigma), so they run side by side on three streams; the
-// forks and joins become edges of the step's graph in captured loops.  A small
-// grid's sweeps leave most of the chip idle alone (32^3 62 -> 48 us per step),
-// a large one's fill each other's last wave (136x88x120 0.855 -> 0.820 ms, PPM
-// 128^3 1.05 -> 1.04, mixed 0.59 -> 0.57, AMR 64 / 720 leaves of 16^3 222 -> 210 us
-// / 1.89 -> 1.87 ms).  The extended-option kernels share the slope array.
+// The three sweeps of a step.  The sweep kernels share only what they read
+// (state and sigma), so they run side by side on three streams; the forks and
+// joins become edges of the step's graph in captured loops.  A small grid's
+// sweeps leave most of the chip idle alone (32^3 62 -> 48 us per step), a large
+// one's fill each other's last wave (136x88x120 0.855 -> 0.820 ms, PPM 128^3
+// 1.05 -> 1.04, mixed 0.59 -> 0.57, AMR 64 / 720 leaves of 16^3 222 -> 210 us /
+// 1.89 -> 1.87 ms).  The per-stage kernels share the slope array.
 //
 // CTAs of two kernels share an SM only under the same split of its memory
 // between L1 and shared memory, and the driver picks each kernel's.  Sweeps
@@ -1245,19 +1268,19 @@ struct SweepStreams {
 };
 template <class R, bool AMR> void launch_sweeps3d(const Args3D &a, dim3 g, cudaStream_t s, const SweepStreams &st)
 {
-    if (extended_options(a.prm)) {
-        launch_states3d<R, AMR, 0>(a, g, false, s);
-        launch_states3d<R, AMR, 1>(a, g, false, s);
-        launch_states3d<R, AMR, 2>(a, g, false, s);
+    if (sweep_form<R>(a) != SWEEP_KERNELS) {
+        launch_stages3d<R, AMR, 0>(a, g, s);
+        launch_stages3d<R, AMR, 1>(a, g, s);
+        launch_stages3d<R, AMR, 2>(a, g, s);
         return;
     }
     const bool max_smem = !(AMR && sizeof(R) == 4) &&
                           (a.prm.order == 5 ? sweep_waves<R, 5, AMR>(a, g.y) : sweep_waves<R, 3, AMR>(a, g.y)) <= 1.5;
     cudaEventRecord(st.fork, s);
     for (int q = 0; q < 2; q++) cudaStreamWaitEvent(st.side[q], st.fork, 0);
-    launch_states3d<R, AMR, 0>(a, g, max_smem, s);
-    launch_states3d<R, AMR, 1>(a, g, max_smem, st.side[0]);
-    launch_states3d<R, AMR, 2>(a, g, max_smem, st.side[1]);
+    launch_one_sweep3d<R, AMR, 0>(a, g.y, max_smem, s);
+    launch_one_sweep3d<R, AMR, 1>(a, g.y, max_smem, st.side[0]);
+    launch_one_sweep3d<R, AMR, 2>(a, g.y, max_smem, st.side[1]);
     for (int q = 0; q < 2; q++) {
         cudaEventRecord(st.join[q], st.side[q]);
         cudaStreamWaitEvent(s, st.join[q], 0);
@@ -1318,7 +1341,7 @@ inline size_t hyb3d_bytes(int nx, int ny, int nz, size_t rsz)
 template <class R> void launch_hydro3d_t(const Args3D &a0, cudaStream_t s, const SweepStreams &st)
 {
     Args3D a = with_divisors(a0, sflux_halo<R>(a0));
-    set_pw_slots<R>(a);
+    set_pw_slots<R>(a, sweep_form<R>(a));
     const int nsig = a.cta[0], nst = a.cta[1], nupd = a.cta[3];
     if (a.prm.use_hybrid) {
         R *divu = (R *)a.hyb;
@@ -1443,7 +1466,7 @@ template <class R> void launch_amr3d_correct_t(const Args3D &a, int entries, con
 template <class R> void launch_amr3d_update_t(const Args3D &a0, int entries, cudaStream_t s)
 {
     Args3D a = with_divisors(a0);
-    set_pw_slots<R>(a);
+    set_pw_slots<R>(a, sweep_form<R>(a));
     update3d_kernel<R, true><<<dim3(a.cta[3], entries), 256, 0, s>>>(a);
 }
 

@@ -10,6 +10,7 @@ cudaError_t setup_hydro3d_mixed() { return cudaSuccess; }
 void launch_hydro3d_mixed(const Args3D &a, cudaStream_t s, const SweepStreams &st) { launch_hydro3d_t<float>(a, s, st); }
 void launch_amr3d_fluxes_mixed(const Args3D &a, int entries, int which, cudaStream_t s, const SweepStreams &st)
 { launch_amr3d_fluxes_t<float>(a, entries, which, s, st); }
+SweepForm hydro3d_form_mixed(const Args3D &a) { return sweep_form<float>(a); }
 void launch_amr3d_emit_mixed(const Args3D &a, int entries, void *bflux, long nfc, cudaStream_t s)
 { launch_amr3d_emit_t<float>(a, entries, bflux, nfc, s); }
 void launch_amr3d_correct_mixed(const Args3D &a, int entries, const void *bflux, long nfc, const int *fine,

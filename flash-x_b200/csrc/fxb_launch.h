@@ -19,6 +19,8 @@ void launch_gravity_faces_mixed(const DevParams &p, void *out, cudaStream_t s);
 cudaError_t setup_hydro3d_mixed();
 void launch_hydro3d_fp64(const Args3D &a, cudaStream_t s, const SweepStreams &st);
 void launch_hydro3d_mixed(const Args3D &a, cudaStream_t s, const SweepStreams &st);
+SweepForm hydro3d_form_fp64(const Args3D &a);
+SweepForm hydro3d_form_mixed(const Args3D &a);
 void launch_amr3d_fluxes_fp64(const Args3D &a, int entries, int which, cudaStream_t s, const SweepStreams &st);
 void launch_amr3d_emit_fp64(const Args3D &a, int entries, void *bflux, long nfc, cudaStream_t s);
 void launch_amr3d_correct_fp64(const Args3D &a, int entries, const void *bflux, long nfc, const int *fine,

@@ -103,6 +103,27 @@ def test_3d_sweep_extents_match_oracle(oracle, need_gpu, shape, order):
         _check(*_steps(oracle, geom, hp, S.noisy_gas(geom, hp)))
 
 
+# FP64 WENO5 with either set of kernels (the tuner would choose by time)
+WENO_3D = {k: OPTIONS_3D[k] for k in ("weno", "weno_primitive", "weno_z", "weno_HLL", "weno_gravity")}
+WENO_3D.update(weno_no_ctu={"order": 5, "use_3dFullCTU": False}, weno_flattening={"order": 5, "use_flattening": True},
+               weno_pressure={"order": 5, "hy_fPresInMomFlux": 0.5})
+
+
+@pytest.mark.parametrize("stages", ["0", "1"])
+@pytest.mark.parametrize("name", sorted(WENO_3D))
+def test_3d_weno_kernels_match_oracle(oracle, need_gpu, monkeypatch, name, stages):
+    monkeypatch.setenv("FXB_WENO_STAGES", stages)
+    geom = Geometry(3, 8, 8, 8, 3, 2, 1,
+                    bc=(BC_REFLECTING, BC_OUTFLOW, BC_PERIODIC, BC_PERIODIC, BC_REFLECTING, BC_REFLECTING))
+    hp = dataclasses.replace(HydroParams(gamma=5.0 / 3.0), **WENO_3D[name])
+    unk = S.noisy_gas(geom, hp)
+    dev = HydroDevice(geom, hp)
+    dev.attach_unk(unk.copy())
+    assert ("sweeps: per-stage kernels" if stages == "1" else "sweeps: one kernel per direction") in dev.tuning()
+    dev.close()
+    _check(*_steps(oracle, geom, hp, unk))
+
+
 def _amr(oracle, geom, hp, maxlev=2, n=2, precisions=("fp64", "mixed")):
     """n steps of the level-set problem: (interiors per precision, oracle's, the last device's tuning text)."""
     mesh, unk = A.levelset_problem(geom, hp, maxlev)
@@ -144,10 +165,11 @@ def test_amr_option_matches_oracle(oracle, need_gpu, monkeypatch, name, persiste
 
 # leaves that fill the sweeps' CTAs of 64, 96, 128 and 160 threads and ones
 # that leave a remainder
-@pytest.mark.parametrize("order", [3, 5])
+@pytest.mark.parametrize("order,stages", [(3, "0"), (5, "0"), (5, "1")])
 @pytest.mark.parametrize("n", [4, 6, 8, 10, 12, 16])
-def test_amr_leaf_sizes_match_oracle(oracle, need_gpu, monkeypatch, n, order):
+def test_amr_leaf_sizes_match_oracle(oracle, need_gpu, monkeypatch, n, order, stages):
     monkeypatch.setenv("FXB_AMR_PERSISTENT", "0")
+    monkeypatch.setenv("FXB_WENO_STAGES", stages)
     geom = Geometry(3, n, n, n, 2, 1, 2, bc=(BC_PERIODIC,) * 2 + (BC_OUTFLOW,) * 2 + (BC_REFLECTING,) * 2)
     _check(*_amr(oracle, geom, HydroParams(order=order))[:2])
 
