@@ -245,13 +245,18 @@ def test_tma_window_equals_thread_loads(need_gpu, monkeypatch, precision):
 
 
 @pytest.mark.parametrize("precision", ["fp64", "mixed"])
-@pytest.mark.parametrize("config", ["rt3d", "sweep3d"])
+@pytest.mark.parametrize("config", ["rt3d", "sweep3d", "rt3d Roe", "sweep3d Roe"])
 def test_ug_launch_shapes_give_identical_states(need_gpu, monkeypatch, precision, config):
     """The uniform-grid tuner only changes launch shapes: the defaults
     (FXB_UG_TUNE=0), the tuned shapes and forced odd ones (CTAs per SM per
     stage, lines per fused face-state tile) step to the same state bit for
-    bit, and fxb_tuning reports the shapes in use."""
-    geom, hp, init = S.config(config, scale=0.25 if config == "rt3d" else 0.5)
+    bit, and fxb_tuning reports the shapes.  The sweep kernels of the default
+    options choose their own grids and read the counts of sigma and update
+    only; Roe's per-stage kernels (FP64) and tiles (FP32) read all of them."""
+    name, _, solver = config.partition(" ")
+    geom, hp, init = S.config(name, scale=0.25 if name == "rt3d" else 0.5)
+    if solver:
+        hp.RiemannSolver = solver
     unk = init(geom, hp)
     outs = []
     for env in ({"FXB_UG_TUNE": "0"}, {}, {"FXB_UG_CTA": "2,16,4,1", "FXB_UG_T1": "1,16,2"}):
