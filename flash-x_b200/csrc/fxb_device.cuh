@@ -69,9 +69,11 @@ template <> __device__ __forceinline__ double rdiv_y<double>(double a, double b,
 }
 template <> __device__ __forceinline__ float rdiv_y<float>(float a, float b, float y) { return a * y; }
 // y = 1 / b for rdiv_y.  FP32: the hardware reciprocal (PTX rcp.approx.ftz.f32,
-// error at most 1 ulp), so that a quotient is within the 2 ulp of the fast
-// division (PTX div.approx.f32) at one multiplication instead of a reciprocal,
-// a multiplication and the scaling of large denominators each.
+// error at most 1 ulp, subnormal results flushed), so that a quotient is one
+// multiplication instead of a reciprocal, a multiplication and the scaling of
+// large denominators each.  With the product's rounding it is within 3 ulp in
+// the worst case (1.5 * 2^-23 relative); whole steps are as far from the FP64
+// path as with the fast division (PTX div.approx.f32, 2 ulp).
 template <class R> __device__ __forceinline__ R rcp_y(R b);
 template <> __device__ __forceinline__ double rcp_y<double>(double b) { return 1.0 / b; }
 template <> __device__ __forceinline__ float rcp_y<float>(float b)
@@ -101,7 +103,7 @@ template <> __device__ __forceinline__ float rsqrt_<float>(float a)
 // FMA and a third step returns RN(1/b) unless b's significand is all ones
 // (P. Markstein, IBM J. Res. Dev. 34(1), 1990; tests/test_reciprocal.py).  A
 // group with a value outside 2^-400 .. 2^400, or with such a significand,
-// takes the division operator.  RT 128^3 FP64 1.63 -> 1.55 ms per step; the
+// takes the division operator.  RT 128^3 FP64 1.63 -> 1.61 ms per step; the
 // eigensystem's and the Riemann solver's divisions, which are not the chain
 // their kernels wait for, got slower this way (KH 2048^2 0.93 -> 0.99 ms).
 __device__ __forceinline__ double rcp64(double b)

@@ -60,9 +60,10 @@ struct Args3D {
     DevParams prm;
     unsigned long long *rate_max;
     int *err;
-    void *sig;      // [3][6][(nx+2)(ny+2)(nz+2)] of R
-    void *wst[3];   // per direction [2][cells with that coordinate in [-1, n]]: Wp, Wm pressures
-    void *flx[3];   // per direction [8][faces]
+    void *sig;      // 18 values of R (sigma_x, sigma_y, sigma_z) per cell of the padded box, tiled (tile_at)
+    void *wst[3];   // per direction, cells with that coordinate in [-1, n]: the two pressures (slots pw_wp,
+                    // pw_wm), or from states3d_kernel all twelve values of Wp and Wm
+    void *flx[3];   // per direction, 8 values per face, tiled (tile_at)
     void *slp;      // PPM: characteristic-limited slopes of the current direction [6][Grid3::ns(d)]
     long slp_bstride;           // AMR: elements of R per batch entry
     void *flat;     // flattening coefficients [3][(nx+2)(ny+2)(nz+2)] of R

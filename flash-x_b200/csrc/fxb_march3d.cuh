@@ -17,12 +17,12 @@
 //
 // Against slope, face-state and flux kernels (FP64) and the fused tile kernel
 // with two barriers per cell (FP32), 128^3: one direction of PPM FP64 374 ->
-// 257 us along y and z and 398 -> 332 us along x, of WENO5 FP64 470 -> 425 and
-// 456 us, PPM FP32 190 -> 128 and 168 us; without the copies ahead the y and z
+// 249 us along y and z and 398 -> 324 us along x, of WENO5 FP64 470 -> 407 to 419
+// and 467 us, PPM FP32 190 -> 123 and 162 us; without the copies ahead the y and z
 // kernels took 390 us.  Whole steps, with the rest of the step as it is now
-// (sweeps side by side, boundary fluxes from here): PPM 1.40 -> 1.04 ms (mixed
-// 0.73 -> 0.57), WENO5 with gravity 1.61 -> 1.52 (mixed 0.76 -> 0.65), AMR (720
-// leaves of 16^3) 2.32 -> 1.87 (mixed 1.25 -> 0.96).
+// (sweeps side by side, boundary fluxes from here): PPM 1.36 -> 1.04 ms (mixed
+// 0.77 -> 0.56), WENO5 with gravity 1.58 -> 1.49 (mixed 0.82 -> 0.61), AMR (288
+// leaves of 16^3) 0.99 -> 0.82 (mixed 0.55 -> 0.43).
 #pragma once
 #include "fxb_hydro3d.cuh"
 #include "fxb_tma.cuh"
@@ -397,9 +397,9 @@ template <class R, int T> constexpr int swx_resident() { return (sizeof(R) == 8 
 // cells per line and tile beyond its faces: one more face state, and with PPM two more slopes
 template <int ORDER> constexpr int swx_extra() { return ORDER == 3 ? 3 : 1; }
 // FP64 copies the sigmas of the next plane into shared memory while it works
-// on this one (RT 128^3 1.55 -> 1.51 ms per step, AMR 16^3 blocks 2.08 -> 2.01);
-// FP32, with five CTAs per SM to switch between, reads them when it needs
-// them (RT 128^3 0.69 ms, 0.71 with the copies)
+// on this one (RT 128^3 1.55 -> 1.51 ms per step, AMR 16^3 blocks 2.08 -> 2.01,
+// before the sweeps ran side by side); FP32, with five CTAs per SM to switch
+// between, reads them when it needs them (RT 128^3 0.69 ms then, 0.71 with the copies)
 template <class R> constexpr bool swx_ahead() { return sizeof(R) == 8; }
 
 template <class R, int ORDER, bool AMR, int OPT, int T>
