@@ -681,27 +681,49 @@ __device__ __forceinline__ void weno_scalar(int method, R I0, R I1, R I2, R I3, 
 template <class R>
 __device__ __noinline__ WenoPair<R> weno_scalar_body(int method, R I0, R I1, R I2, R I3, R I4)
 {
-    const R c6 = R(6.);
-    const R p00 = R(2.) / c6, p01 = R(-7.) / c6, p02 = R(11.) / c6;
-    const R p10 = R(-1.) / c6, p11 = R(5.) / c6, p12 = R(2.) / c6;
-    const R p20 = R(2.) / c6, p21 = R(5.) / c6, p22 = R(-1.) / c6;
-    const R m00 = R(-1.) / c6, m01 = R(5.) / c6, m02 = R(2.) / c6;
-    const R m10 = R(2.) / c6, m11 = R(5.) / c6, m12 = R(-1.) / c6;
-    const R m20 = R(11.) / c6, m21 = R(-7.) / c6, m22 = R(2.) / c6;
-    R w5p0 = p00 * I0 + p01 * I1 + p02 * I2;
-    R w5p1 = p10 * I1 + p11 * I2 + p12 * I3;
-    R w5p2 = p20 * I2 + p21 * I3 + p22 * I4;
-    R w5m0 = m00 * I0 + m01 * I1 + m02 * I2;
-    R w5m1 = m10 * I1 + m11 * I2 + m12 * I3;
-    R w5m2 = m20 * I2 + m21 * I3 + m22 * I4;
-    const R c1312 = R(13.) / R(12.);
-    R t1, t2;
-    t1 = I0 - R(2.) * I1 + I2; t2 = I0 - R(4.) * I1 + R(3.) * I2;
-    R b0 = c1312 * (t1 * t1) + R(0.25) * (t2 * t2);
-    t1 = I1 - R(2.) * I2 + I3; t2 = I1 - I3;
-    R b1 = c1312 * (t1 * t1) + R(0.25) * (t2 * t2);
-    t1 = I2 - R(2.) * I3 + I4; t2 = R(3.) * I2 - R(4.) * I3 + I4;
-    R b2 = c1312 * (t1 * t1) + R(0.25) * (t2 * t2);
+    const R c6 = R(6.), c1312 = R(13.) / R(12.);
+    // the candidates at i + 1/2 and i - 1/2 and the smoothness indicators
+    R w5p0, w5p1, w5p2, w5m0, w5m1, w5m2, b0, b1, b2, t1, t2;
+    if constexpr (sizeof(R) == 4) {
+        // from the four differences, the candidates less the cell's own value:
+        // the rounding of coefficients, products and weights is then relative
+        // to differences, and only the last sum rounds at the value's size
+        // (0.23 instead of 0.60 ulp rms for a stencil around 1; the velocity error
+        // of mixed steps 7 % lower, WENO5 128^3 610 -> 604 us per step)
+        const R da = I0 - I1, db = I1 - I2, dc = I2 - I3, dd = I3 - I4;
+        const R k1 = R(1.) / c6, k2 = R(2.) / c6, k4 = R(4.) / c6, k5 = R(5.) / c6;
+        w5p0 = k2 * da - k5 * db;
+        w5p1 = -k1 * db - k2 * dc;
+        w5p2 = k1 * dd - k4 * dc;
+        w5m0 = k4 * db - k1 * da;
+        w5m1 = k2 * db + k1 * dc;
+        w5m2 = k5 * dc - k2 * dd;
+        t1 = da - db; t2 = da - R(3.) * db;
+        b0 = c1312 * (t1 * t1) + R(0.25) * (t2 * t2);
+        t1 = db - dc; t2 = db + dc;
+        b1 = c1312 * (t1 * t1) + R(0.25) * (t2 * t2);
+        t1 = dc - dd; t2 = R(3.) * dc - dd;
+        b2 = c1312 * (t1 * t1) + R(0.25) * (t2 * t2);
+    } else {
+        const R p00 = R(2.) / c6, p01 = R(-7.) / c6, p02 = R(11.) / c6;
+        const R p10 = R(-1.) / c6, p11 = R(5.) / c6, p12 = R(2.) / c6;
+        const R p20 = R(2.) / c6, p21 = R(5.) / c6, p22 = R(-1.) / c6;
+        const R m00 = R(-1.) / c6, m01 = R(5.) / c6, m02 = R(2.) / c6;
+        const R m10 = R(2.) / c6, m11 = R(5.) / c6, m12 = R(-1.) / c6;
+        const R m20 = R(11.) / c6, m21 = R(-7.) / c6, m22 = R(2.) / c6;
+        w5p0 = p00 * I0 + p01 * I1 + p02 * I2;
+        w5p1 = p10 * I1 + p11 * I2 + p12 * I3;
+        w5p2 = p20 * I2 + p21 * I3 + p22 * I4;
+        w5m0 = m00 * I0 + m01 * I1 + m02 * I2;
+        w5m1 = m10 * I1 + m11 * I2 + m12 * I3;
+        w5m2 = m20 * I2 + m21 * I3 + m22 * I4;
+        t1 = I0 - R(2.) * I1 + I2; t2 = I0 - R(4.) * I1 + R(3.) * I2;
+        b0 = c1312 * (t1 * t1) + R(0.25) * (t2 * t2);
+        t1 = I1 - R(2.) * I2 + I3; t2 = I1 - I3;
+        b1 = c1312 * (t1 * t1) + R(0.25) * (t2 * t2);
+        t1 = I2 - R(2.) * I3 + I4; t2 = R(3.) * I2 - R(4.) * I3 + I4;
+        b2 = c1312 * (t1 * t1) + R(0.25) * (t2 * t2);
+    }
     const R tiny = R(1.e-36);
     // every quotient below shares its denominator with another: the
     // indicators' with the other side's, the sums' with the other weights
@@ -723,15 +745,9 @@ __device__ __noinline__ WenoPair<R> weno_scalar_body(int method, R I0, R I1, R I
     const R s[2] = {a[0] + a[1] + a[2], c[0] + c[1] + c[2]};
     R ys[2];
     recips(s, ys);
-    if constexpr (sizeof(R) == 4) {
-        // the middle weight as one minus the other two: the rounding of the
-        // weights then multiplies differences of the candidates and not the
-        // candidates themselves
-        return WenoPair<R>{w5p1 + rdiv_y(a[0], s[0], ys[0]) * (w5p0 - w5p1) + rdiv_y(a[2], s[0], ys[0]) * (w5p2 - w5p1),
-                           w5m1 + rdiv_y(c[0], s[1], ys[1]) * (w5m0 - w5m1) + rdiv_y(c[2], s[1], ys[1]) * (w5m2 - w5m1)};
-    }
     const R vr = rdiv_y(a[0], s[0], ys[0]) * w5p0 + rdiv_y(a[1], s[0], ys[0]) * w5p1 + rdiv_y(a[2], s[0], ys[0]) * w5p2;
     const R vl = rdiv_y(c[0], s[1], ys[1]) * w5m0 + rdiv_y(c[1], s[1], ys[1]) * w5m1 + rdiv_y(c[2], s[1], ys[1]) * w5m2;
+    if constexpr (sizeof(R) == 4) return WenoPair<R>{I2 + vr, I2 + vl};
     return WenoPair<R>{vr, vl};
 }
 
